@@ -253,6 +253,7 @@ void free_all(Ctx& c) {
   block_free(c);
   if (c.d_clouds) cudaFree(c.d_clouds);
   if (c.gact) cudaFree(c.gact);
+  if (c.ggrp) cudaFree(c.ggrp);
   void* ps[] = {c.pm, c.hz, c.vel, c.csq, c.orig, c.pm_alt, c.hz_alt, c.vel_alt, c.csq_alt,
                 c.orig_alt, c.rho, c.omega, c.div_v, c.drhodt, c.rho_alt, c.omega_alt, c.div_v_alt,
                 c.drhodt_alt, c.press, c.sound, c.acc, c.gpot,
@@ -261,7 +262,7 @@ void free_all(Ctx& c) {
                 c.rs_hist, c.bbox_part, c.branch, c.branch_next, c.nchild, c.choff, c.cstart,
                 c.bflag, c.bscan, c.leaf, c.nextcell, c.ifopen, c.pstart, c.pcount, c.parent,
                 c.level, c.nkids, c.work, c.sinks, c.wstack, c.leaves, c.nleaf, c.npot, c.redo, c.wide, c.wst, c.wacc, c.link, c.gA, c.gB, c.gC, c.wA, c.hN, c.hA, c.hrm, c.hA32, c.hrm32, c.hmax, c.bbmin, c.bbmax, c.d_info,
-                c.d_err, c.d_counts, c.sink_out, c.tabA, c.tabG, c.tabG32, c.scan.total, c.scan.level_buf[0],
+                c.d_err, c.d_counts, c.sink_out, c.tabA, c.tabG, c.scan.total, c.scan.level_buf[0],
                 c.scan.level_buf[1], c.scan.level_buf[2], c.scan.level_buf[3]};
   for (void* p : ps)
     if (p) cudaFree(p);
@@ -317,7 +318,7 @@ int alloc_all(Ctx& c) {
          alloc(c.hmax, C) | alloc(c.bbmin, C) | alloc(c.bbmax, C);
   bad |= alloc(c.d_info, 1) | alloc(c.d_err, 1) | alloc(c.d_counts, 32) | alloc(c.sinks, 5 * 1024) |
          alloc(c.sink_out, 4 * 1024);
-  bad |= alloc(c.tabA, KERNTOT + 1) | alloc(c.tabG, KERNTOT + 1) | alloc(c.tabG32, KERNTOT + 1);
+  bad |= alloc(c.tabA, KERNTOT + 1) | alloc(c.tabG, KERNTOT + 1);
   c.wstack_slots = std::max(grav_walk_slots(c), hydro_walk_slots(c));
   c.wstack_cap = grav_walk_stack_cap(c);
   bad |= alloc(c.wstack, (size_t)c.wstack_slots * c.wstack_cap);
@@ -341,12 +342,6 @@ int alloc_all(Ctx& c) {
   if (cudaMemcpy(c.tabA, ta.data(), sizeof(double4) * ta.size(), cudaMemcpyHostToDevice) != cudaSuccess)
     return -1;
   if (cudaMemcpy(c.tabG, tg.data(), sizeof(double4) * tg.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-    return -1;
-  std::vector<float4> t32(KERNTOT + 1);
-  for (int i = 0; i <= KERNTOT; ++i)
-    t32[i] = make_float4((float)w5[i], (float)w4[i], (float)w6[i], 0.0f);
-  if (cudaMemcpy(c.tabG32, t32.data(), sizeof(float4) * t32.size(), cudaMemcpyHostToDevice) !=
-      cudaSuccess)
     return -1;
   return 0;
 }
@@ -1196,19 +1191,33 @@ int seren_gpu_set_clouds(seren_gpu_ctx* h, int32_t ncloud, const int32_t* counts
     for (int i = 0; i < cl[k].n; ++i) gl.push_back(cl[k].pstart + i);
     while (gl.size() % 32) gl.push_back(-1);
   }
+  // the gravity walk's groups: each cloud's as wide as when it is alone, its
+  // offset in gact (a multiple of four) and width in one word
+  std::vector<int> gg;
+  size_t off = 0;
+  for (int k = 0; k < ncloud; ++k) {
+    const int lpw = seren::grav_lpw(cl[k].n);
+    for (int i = 0; i < cl[k].n; i += 1 << lpw) gg.push_back((int)((off + i) / 4) * 8 + lpw);
+    off += (size_t)nb(cl[k].n, 32) * 32;
+  }
   if (c.d_clouds) cudaFree(c.d_clouds);
   if (c.gact) cudaFree(c.gact);
+  if (c.ggrp) cudaFree(c.ggrp);
   c.d_clouds = nullptr;
   c.gact = nullptr;
+  c.ggrp = nullptr;
   if (cudaMalloc(&c.d_clouds, sizeof(seren::CloudInfo) * ncloud) != cudaSuccess ||
-      cudaMalloc(&c.gact, sizeof(int) * gl.size()) != cudaSuccess) {
+      cudaMalloc(&c.gact, sizeof(int) * gl.size()) != cudaSuccess ||
+      cudaMalloc(&c.ggrp, sizeof(int) * gg.size()) != cudaSuccess) {
     cudaGetLastError();
     return fail(c, SEREN_GPU_ERR_CUDA, "set_clouds: allocation failed");
   }
   cudaMemcpyAsync(c.d_clouds, cl.data(), sizeof(seren::CloudInfo) * ncloud, cudaMemcpyHostToDevice, c.st);
   cudaMemcpyAsync(c.gact, gl.data(), sizeof(int) * gl.size(), cudaMemcpyHostToDevice, c.st);
+  cudaMemcpyAsync(c.ggrp, gg.data(), sizeof(int) * gg.size(), cudaMemcpyHostToDevice, c.st);
   c.clouds = cl;
   c.ngact = (int)gl.size();
+  c.nggrp = (int)gg.size();
   c.ncloud = ncloud;
   return finish(c, "set_clouds");
 }

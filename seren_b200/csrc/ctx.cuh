@@ -189,7 +189,7 @@ struct Ctx {
   bool gsets = false;             // the last grad-h recorded the gather neighbours (launch_neib)
   int* wcover = nullptr;          // the cells their walks are spread over (made on first use)
   int wcover_cap = 0;
-  double4* hrec = nullptr;        // hydro: 96-byte neighbour records, 3 per particle (first use)
+  double4* hrec = nullptr;        // records of the mixed hydro and gravity kernels (hydro_records)
   int2* wstack = nullptr;     // walk stacks, wstack_cap (cell, lane mask) entries per warp slot
   int wstack_cap = 0;
   int wstack_slots = 0;
@@ -197,7 +197,6 @@ struct Ctx {
   // kernel tables
   double4* tabA = nullptr;
   double4* tabG = nullptr;
-  float4* tabG32 = nullptr;   // FP32 w5, w4, w6 of tabG (mixed gravity)
 
   // sink accretion and search (seren_gpu_accrete, seren_gpu_sink_search), made
   // on first use: sink records and results, ACC_STRIDE doubles per sink for up
@@ -218,6 +217,8 @@ struct Ctx {
   CloudInfo* d_clouds = nullptr;
   int* gact = nullptr;
   int ngact = 0;
+  int* ggrp = nullptr;                 // the gravity walk's groups over gact (launch_grav)
+  int nggrp = 0;
 
   // build schedule of the device-resident force steps (main/tree_update.F90:
   // build every nbuildstep evaluations, restock in between)
@@ -282,6 +283,10 @@ void launch_hgather(Ctx& c, int nact);  // h_gather (standard SPH)
 void launch_neib(Ctx& c, int nact, bool sorted = true);
 void launch_hydro(Ctx& c, int nact, double* amap = nullptr);   // amap: mapped host a (optional)
 void launch_thermal(Ctx& c);
+// c.hrec, 96 bytes per particle, made on first use: the neighbour records of the
+// mixed hydro kernel, then the near-field records of the mixed gravity walk (each
+// written and read on c.st); 0, or -1 with the error flagged on the device
+int hydro_records(Ctx& c);
 int hydro_walk_slots(const Ctx& c);     // resident warps of the grad-h / neighbour grids
 int wide_scratch_alloc(Ctx& c);         // c.wst, c.wacc; 0 or -1
 // check_neighbour_timesteps: every active particle's level reaches the
@@ -295,6 +300,7 @@ void launch_neib_levels(Ctx& c, int nact, const int* nlevel, int* nminneib);
 void launch_grav(Ctx& c, int nact, int nsink, const double* d_sinks, double* amap = nullptr,
                  double* gmap = nullptr, const double* abase = nullptr);
 void launch_sink_walk(Ctx& c, int nsink, const double* d_sinks, double* d_out /*[nsink][4]*/);
+int grav_lpw(int n);                    // log2 of the particles per gravity walk group
 int grav_walk_slots(const Ctx& c);      // resident warps of the gravity walk grid
 int grav_walk_stack_cap(const Ctx& c);  // stack entries per warp
 

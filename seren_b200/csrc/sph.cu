@@ -2606,16 +2606,18 @@ static void launch_neib_gsets(Ctx& c, bool sorted) {
   c.nlaunch += 2;
 }
 
+int hydro_records(Ctx& c) {
+  if (c.hrec) return 0;
+  if (cudaMalloc(&c.hrec, sizeof(double4) * 3 * (size_t)c.pmax) == cudaSuccess) return 0;
+  cudaGetLastError();
+  c.hrec = nullptr;
+  k_flag_error<<<1, 1, 0, c.st>>>(c.d_err, SEREN_GPU_ERR_CUDA, KID_HYDRO);
+  return -1;
+}
+
 void launch_hydro(Ctx& c, int nact, double* amap) {
   if (nact <= 0) return;
-  if (c.prm.precision != 0 && !c.hrec) {        // made on first use
-    if (cudaMalloc(&c.hrec, sizeof(double4) * 3 * (size_t)c.pmax) != cudaSuccess) {
-      cudaGetLastError();
-      c.hrec = nullptr;
-      k_flag_error<<<1, 1, 0, c.st>>>(c.d_err, SEREN_GPU_ERR_CUDA, KID_HYDRO);
-      return;
-    }
-  }
+  if (c.prm.precision != 0 && hydro_records(c)) return;
   if (c.prm.precision != 0)
     k_hydro_prep_pack<<<nb(c.ptot, 256), 256, 0, c.st>>>(c.ptot, c.pm, c.hz, c.vel, c.rho,
                                                          c.omega, c.press, c.sound, c.pf, c.hf4,
