@@ -18,6 +18,7 @@
 
 #include "ctx.cuh"
 #include "kernel_fns.h"
+#include "warp.cuh"
 
 namespace seren {
 
@@ -417,6 +418,13 @@ __device__ __forceinline__ double warp_sum(double v) {
   return __shfl_sync(FULL, v, 0);
 }
 
+// A work counter grows by the warp's sum of v: one atomic per warp, since the
+// lanes' own, all to one address, took 0.25 ms of a kernel's end.
+__device__ __forceinline__ void warp_count(unsigned long long* c, unsigned v, int lane) {
+  const unsigned n = __reduce_add_sync(FULL, v);
+  if (lane == 0) atomicAdd(c, (unsigned long long)n);
+}
+
 __device__ __forceinline__ int gr_next(int* work, int lane) {
   int g = 0;
   if (lane == 0) g = atomicAdd(work, 1);
@@ -426,39 +434,59 @@ __device__ __forceinline__ int gr_next(int* work, int lane) {
 // sph/all_sph_gradh.F90:11-492 in two kernels.
 //
 // k_gradh_walk: the first neighbour walk of every active particle
-// (:154-170, BHhydrowalk_hgather at h_high = h*HMULT), 32 particles per warp
-// on a group walk; each particle's opened leaves go to its own row of
-// c.leaves (GH_LEAVES codes pstart*8 + count-1, in walk order) and their
-// number to c.nleaf (-1 when the row or the walk overflows).
+// (:154-170, BHhydrowalk_hgather at h_high = h*HMULT), one group walk per warp;
+// the particles of the opened leaves are then tested against every particle of
+// the group at once, and each particle's candidates within 2 h_high (a superset,
+// FP32 with a margin) go to its own row of c.leaves (GH_LEAVES ids, in leaf
+// order), their number to c.nleaf (-1 when the row or the walk overflows), the
+// number of particles in the leaves it opened (pp_pot) to c.npot.
 //
-// k_gradh_pass: 32 particles per warp, each lane holding its particle's state;
-// the reference's iteration (:154-285) and final pass (:317-425) run with the
-// candidates of one particle at a time (its row flattened) shared out over the
-// lanes and the sums reduced across the warp.  The reference leaves this path
-// only to grow h (pp_pot < pp_gather) or to walk again (h > h_high); a
-// particle that needs either, or whose row overflowed, is redone from the
-// start with walks of its own, which take the reference's steps in the same
-// order: k_gradh_redo (one warp per particle, walk buffers in global scratch)
-// and, for walks too large for those buffers, k_gradh_wide (one block per
-// particle, walks split over subtrees).
-constexpr int GH_LEAVES = 256;   // opened leaves kept per particle
+// k_gradh_pass: each lane holds one particle's state; the reference's iteration
+// (:154-285) and final pass (:317-425) run over the recorded candidates, which
+// hold every particle within 2h while h <= h_high.  The reference leaves this
+// path only to grow h (pp_pot < pp_gather) or to walk again (h > h_high); a
+// particle that needs either, whose final h reaches h_high, or whose row
+// overflowed, is redone from the start with walks of its own, which take the
+// reference's steps in the same order: k_gradh_redo (one warp per particle, walk
+// buffers in global scratch) and, for walks too large for those buffers,
+// k_gradh_wide (one block per particle, walks split over subtrees).
+constexpr int GH_LEAVES = 256;   // candidates (or, for the neighbour walk, leaves) per particle
+constexpr int GH_B = 64;         // particles of opened leaves tested at a time
+constexpr int GH_LS = GH_B + 4;  // list stride: an odd number of words
 
+// k_gradh_walk's per-warp shared state beside the walk's
+struct GhShared {
+  GrShared w;
+  float x[GH_B], y[GH_B], z[GH_B];   // a batch: positions relative to the group's first particle
+  int id[GH_B];
+  unsigned char pick[32 * GH_LS];    // each particle's candidates of the batch
+  int cnt[32], tot[32], p[32];
+};
+
+// groups, lpw: as k_grav_walk (a group of 2^lpw particles per warp)
 __global__ void __launch_bounds__(GR_THREADS) k_gradh_walk(
-    int nact, const int* __restrict__ act, const double4* __restrict__ pm,
-    const double2* __restrict__ hz, HydroTree t, int* __restrict__ leaves,
-    int* __restrict__ nleaf, int* __restrict__ npot, int2* __restrict__ stacks, int scap,
+    int nact, const int* __restrict__ act, int ngroups, const int* __restrict__ groups, int lpw,
+    const double4* __restrict__ pm,
+    const double2* __restrict__ hz, HydroTree t, int* __restrict__ rows,
+    int* __restrict__ nrow, int* __restrict__ npot, int2* __restrict__ stacks, int scap,
     unsigned long long* counts, int* work) {
   extern __shared__ __align__(16) unsigned char gr_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  GrShared& R = reinterpret_cast<GrShared*>(gr_smem)[w];
+  GhShared& H = reinterpret_cast<GhShared*>(gr_smem)[w];
+  GrShared& R = H.w;
   int2* const S = stacks + (size_t)(blockIdx.x * GR_WARPS + w) * scap;
-  const unsigned bit = 1u << lane;
   unsigned long long nvisit = 0;
   unsigned nwalk = 0;
-  for (int g = gr_next(work, lane); (long long)g * 32 < nact; g = gr_next(work, lane)) {
-    const int i = g * 32 + lane;
+  for (int g = gr_next(work, lane); g < ngroups; g = gr_next(work, lane)) {
+    int i0 = g << lpw;
+    if (groups) {
+      const int code = groups[g];
+      i0 = (code >> 3) * 4;
+      lpw = code & 7;
+    }
+    const int PW = 1 << lpw;
     bool live;
-    const int p = group_particle(i, nact, act, live);
+    const int p = group_particle(i0 + (lane & (PW - 1)), nact, act, live);
     const TreeFrame fr = frame_for(t, p);             // lanes share one cloud
     const double4 P = pm[p];
     const double rx = P.x, ry = P.y, rz = P.z;
@@ -466,7 +494,7 @@ __global__ void __launch_bounds__(GR_THREADS) k_gradh_walk(
     const double Rw = KERNRANGE * (hz[p].x * HMULT);                  // :157-158
     const float R32 = (float)Rw;
     const unsigned lanes = __ballot_sync(FULL, live);
-    nwalk += live ? 1u : 0u;
+    nwalk += live && lane < PW ? 1u : 0u;
     const GrGroup grp = gr_group(px, py, pz, R32, live);
     const int nent = gr_walk(t, fr.root, lanes, S, scap, R, lane, 0, nvisit, [&](const float4& c, float) {
       return gr_decide(grp, c, grp.rmin, grp.rmax, fr.delta);
@@ -482,25 +510,126 @@ __global__ void __launch_bounds__(GR_THREADS) k_gradh_walk(
     });
     int n = -1, pot = 0;
     if (nent >= 0) {
-      n = 0;
-      int* row = leaves + (size_t)p * GH_LEAVES;
-      for (int e = 0; e < nent; ++e) {
-        if (R.mask[e] & bit) {
-          const int code = R.code[e];
-          if (n < GH_LEAVES) row[n] = code;
-          ++n;
-          pot += (code & 7) + 1;                        // pp_pot, :168
-        }
+      // pp_pot (:168): the counts of the leaves each lane opened, 32 leaves at a
+      // time from their masks transposed and the bits of their counts
+      for (int e = lane; e - lane < nent; e += 32) {
+        const int c1 = e < nent ? R.code[e] & 7 : 0;
+        const unsigned wd = warp_transpose(e < nent ? R.mask[e] : 0u, lane);
+        pot += __popc(wd) + __popc(wd & __ballot_sync(FULL, c1 & 1)) +
+               2 * __popc(wd & __ballot_sync(FULL, c1 & 2)) +
+               4 * __popc(wd & __ballot_sync(FULL, c1 & 4));
       }
+      // this lane's particle relative to the group's first one, and its radius
+      // 2 h_high with a margin for the rounding of either offset (2^-24 of a
+      // candidate's, itself at most this lane's plus the radius, and of the
+      // difference and the squares)
+      const double fx = __shfl_sync(FULL, rx, 0), fy = __shfl_sync(FULL, ry, 0),
+                   fz = __shfl_sync(FULL, rz, 0);
+      const float ux = (float)(rx - fx), uy = (float)(ry - fy), uz = (float)(rz - fz);
+      const float um = fabsf(ux) + fabsf(uy) + fabsf(uz);
+      const float Rm = fmaf(2.0e-6f, um + R32, R32) * 1.000002f;
+      const float T = live ? Rm * Rm * 1.000002f : -1.0f;
+      const f2 nx = pk1(-ux), ny = pk1(-uy), nz = pk1(-uz), nT = pk1(-T);
+      if (lane < PW) {
+        H.tot[lane] = 0;
+        H.p[lane] = p;
+      }
+      // the opened leaves' particles, in batches
+      int nb = 0, l0 = 0, done = 0;
+      while (l0 < nent) {
+        __syncwarp();
+        int code = 0, cnt = 0;
+        if (l0 + lane < nent) {
+          code = R.code[l0 + lane];
+          cnt = (code & 7) + 1;
+        }
+        const int inc = warp_iscan(cnt, lane);
+        const unsigned fit = __ballot_sync(FULL, inc > done && inc - done <= GH_B - nb);
+        const int upto = fit ? __shfl_sync(FULL, inc, 31 - __clz(fit)) : done;
+        if ((fit >> lane) & 1u) {
+          const int o = nb + inc - done - cnt;
+          for (int q = 0; q < cnt; ++q) H.id[o + q] = (code >> 3) + q;
+        }
+        nb += upto - done;
+        done = upto;
+        const bool all = done == __shfl_sync(FULL, inc, 31);
+        if (all) {
+          l0 += 32;
+          done = 0;
+          if (l0 < nent) continue;                     // more leaves into this batch
+        }
+        // the batch is full, or the list done: every lane tests each particle
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < GH_B / 32; ++u) {
+          const int e = 32 * u + lane;
+          float x = 3.0e38f, y = 3.0e38f, z = 3.0e38f;
+          if (e < nb) {
+            const double4 Q = pm[H.id[e]];
+            x = (float)(Q.x - fx);
+            y = (float)(Q.y - fy);
+            z = (float)(Q.z - fz);
+          }
+          H.x[e] = x;
+          H.y[e] = y;
+          H.z[e] = z;
+        }
+        __syncwarp();
+        int np = 0;
+        unsigned char* row = H.pick + (lane & (PW - 1)) * GH_LS;
+#pragma unroll 1
+        for (int c = 0; c < nb; c += 32) {
+          unsigned wd = 0u;
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            const float4 X = *reinterpret_cast<const float4*>(&H.x[c + e]);
+            const float4 Y = *reinterpret_cast<const float4*>(&H.y[c + e]);
+            const float4 Z = *reinterpret_cast<const float4*>(&H.z[c + e]);
+            const f2 ax = add2(pk(X.x, X.y), nx), bx = add2(pk(X.z, X.w), nx);
+            const f2 ay = add2(pk(Y.x, Y.y), ny), by = add2(pk(Y.z, Y.w), ny);
+            const f2 az = add2(pk(Z.x, Z.y), nz), bz = add2(pk(Z.z, Z.w), nz);
+            float d0, d1, d2, d3;
+            // the sign of r^2 - T, shifted in: particle e's bit ends at 31 - e
+            unpk(fma2(az, az, fma2(ay, ay, fma2(ax, ax, nT))), d0, d1);
+            unpk(fma2(bz, bz, fma2(by, by, fma2(bx, bx, nT))), d2, d3);
+            wd = __funnelshift_l(__float_as_uint(d0), wd, 1);
+            wd = __funnelshift_l(__float_as_uint(d1), wd, 1);
+            wd = __funnelshift_l(__float_as_uint(d2), wd, 1);
+            wd = __funnelshift_l(__float_as_uint(d3), wd, 1);
+          }
+          if (lane < PW) {
+            while (wd != 0u) {
+              const int b = __clz(wd);
+              row[np++] = (unsigned char)(c + b);
+              wd ^= 0x80000000u >> b;
+            }
+          }
+        }
+        if (lane < PW) H.cnt[lane] = np;
+        __syncwarp();
+        // to the rows, eight lanes per particle
+        for (int j0 = 0; j0 < PW; j0 += 4) {
+          const int j = j0 + (lane >> 3);
+          const int nj = H.cnt[j], tj = H.tot[j];
+          int* out = rows + (size_t)H.p[j] * GH_LEAVES + tj;
+          for (int k = lane & 7; k < nj; k += 8)
+            if (tj + k < GH_LEAVES) out[k] = H.id[H.pick[j * GH_LS + k]];
+        }
+        __syncwarp();
+        if (lane < PW) H.tot[lane] += np;
+        nb = 0;
+      }
+      __syncwarp();
+      n = lane < PW ? H.tot[lane] : 0;
       if (n > GH_LEAVES) n = -1;
     }
-    if (live) {
-      nleaf[p] = n;
+    if (live && lane < PW) {
+      nrow[p] = n;
       npot[p] = pot;
     }
     __syncwarp();
   }
-  atomicAdd(counts + 3, (unsigned long long)nwalk);
+  warp_count(counts + 3, nwalk, lane);
   if (lane == 0) atomicAdd(counts + 4, nvisit);
 }
 
@@ -554,155 +683,93 @@ __device__ __forceinline__ int gp_flatten(const int* __restrict__ row, int n, in
   return total;
 }
 
-constexpr int GP_PSEG = 32;      // k_gradh_pass: leaves of a row flattened at a time
-constexpr int GP_PINB = 128;     // k_gradh_pass: packed in-range candidates per warp
+// The kernel bin int(5000 r/h) of a pair, y = (r/h)^2, from an FP32 root; sure =
+// false when that lies too close to a bin's edge to tell (its error is below
+// 2e-3 bins; y not a normal FP32 number included) and gh_bin_exact must decide.
+__device__ __forceinline__ int gh_bin(double y, bool& sure) {
+  const float t2 = (float)y * 2.5e7f;
+  const float t = t2 * rsqrt_n(t2);
+  const float tm = __fadd_rd(t, 8388608.0f);
+  const float fr = t - (tm - 8388608.0f);
+  sure = fr >= 4.0e-3f && fr <= 0.996f;
+  return __float_as_int(tm) - 0x4b000000;
+}
+__device__ __noinline__ int gh_bin_exact(double d2, double ih) {
+  return min((int)((HALFKERNTOT * (sqrt(d2) + SMALL_NUMBER)) * ih), 2 * KERNTOT);
+}
+// (double)k for 0 <= k < 2^31
+__device__ __forceinline__ double int_double(int k) {
+  return __hiloint2double(0x43300000, k) - 4503599627370496.0;
+}
+// The M4 kernel of setup/kernel.F90 at the centre s = (2k+1) 1e-4 of bin k, by the
+// whole numbers U = 1e4 (2 - s) and V = 1e4 (1 - s), cut off at zero: with u = 2 - s and v
+// = 1 - s, w0 = (u^3 - 4v^3)/4, w4 = dw0/ds = -3(u^2 - 4v^2)/4, wh = -(3 w0 + s w4)
+// (all times 1/pi), wg = u^4(1/2 - u/5) - v^4(1 - 4v/5).
+__device__ __forceinline__ void gh_uv(int k, double& U, double& V) {
+  U = int_double(max(2 * KERNTOT - 1 - 2 * k, 0));
+  V = int_double(max(KERNTOT - 1 - 2 * k, 0));
+}
 
-template <int N>
-using ICst = std::integral_constant<int, N>;
-
-// k_gradh_pass's per-warp shared state: the group's per-particle values that
-// the candidate loops read for one particle at a time (broadcast loads), a
-// flattened row segment, and the packed in-range candidates.
+// k_gradh_pass's per-warp shared state: the group's per-particle values, which
+// eight lanes read for one particle, and the sums they return.
 struct GpWarp {
   double x[32], y[32], z[32];
-  double hs[32], ih[32], hf[32];   // (2h)^2, 1/h, 1/h^3 of the pass in progress
-  double hh[32];                   // (2 h_high)^2: radius of the recorded candidates
-  int p[32], n[32], npr[32];       // particle, leaves in its row, recorded candidates (-1: none)
-  unsigned cpl;                    // lanes whose final-pass candidates hold every particle within 2h
-  int cand[GP_PSEG * LEAFMAX];
-  double d2[GP_PINB], m[GP_PINB], dv[GP_PINB];
+  double hs[32], ih[32];           // (2h)^2 and 1/h of the pass in progress
+  double part[32][4];
+  int p[32], n[32], g[32];         // particle, candidates, gather neighbours
+  int list[32];                    // the particles of the pass
 };
 
-// 32 consecutive particles per warp: each lane holds its particle's iteration
-// state, so the per-particle arithmetic of a pass (h, its powers, the update
-// of :238-285) runs once per lane for all 32; each particle's candidates are
-// shared out over the 32 lanes in turn, 32*U at a time with all their loads
-// issued together (U = 4 for the recorded candidates of the density passes).
+// Each lane holds its particle's iteration state, so the per-particle
+// arithmetic of a pass (h, its powers, the update of :238-285) runs once per lane;
+// the candidates are shared out over eight lanes per particle, four particles at a
+// time.  A warp takes 2^lpw particles: fewer when there are too few for every
+// resident warp to get 32 (a particle's sums do not depend on it).
+//
+// Bound by the latency of its gathers and FP64 chains.  On a 1M-particle core: 1.45
+// ms (3.13 ms when a warp took one particle at a time, tested every particle of
+// its opened leaves and packed those in range before evaluating them); with
+// k_gradh_walk, which now does the testing (0.92 ms before), 3.0 ms against 4.05.
+// At 32768 particles 82 us against 381 (every lane's own atomics on the work
+// counters were 250 us of that).
+template <int U>
+__device__ __forceinline__ void gp_load(const int* __restrict__ row, int k, int n, int pj,
+                                        const double4* __restrict__ pm, int (&q)[U],
+                                        double4 (&Q)[U]) {
+#pragma unroll
+  for (int u = 0; u < U; ++u) q[u] = k + 8 * u < n ? row[k + 8 * u] : pj;
+#pragma unroll
+  for (int u = 0; u < U; ++u) Q[u] = pm[q[u]];
+}
+
 __global__ void __launch_bounds__(GP_THREADS, 8) k_gradh_pass(
-    int nact, const int* __restrict__ act, const double4* __restrict__ pm, double2* __restrict__ hz,
+    int nact, const int* __restrict__ act, int lpw, const double4* __restrict__ pm,
+    double2* __restrict__ hz,
     const double4* __restrict__ vel, double* __restrict__ rho, double* __restrict__ omega,
     double* __restrict__ divv, double* __restrict__ drhodt, const double4* __restrict__ tabA,
-    double h_fac, int pp_gather, double rextent0, const int* __restrict__ leaves,
-    const int* __restrict__ nleaf, int* __restrict__ npot, int* __restrict__ redo,
-    int* __restrict__ nredo, int* __restrict__ prune, int L, DevError* err,
+    double h_fac, int pp_gather, double rextent0, const int* __restrict__ rows,
+    const int* __restrict__ nrow, int* __restrict__ npot, int* __restrict__ redo,
+    int* __restrict__ nredo, int* __restrict__ gset, int L, DevError* err,
     unsigned long long* counts, int* work, const CloudInfo* __restrict__ cl, int ncl, int rec,
     int* __restrict__ pptot) {
+  constexpr int U = 2, UF = 1;
   __shared__ GpWarp gpw[GP_WARPS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int l8 = lane & 7, quad = lane >> 3;
   GpWarp& W = gpw[w];
   const unsigned lt = (1u << lane) - 1u;
+  const int PW = 1 << lpw;
   unsigned npass = 0, ncands = 0, niter = 0, nsingle = 0;
 
-  // Density sum (:211-235) of particle j over the candidates getq(0..nc): r^2
-  // of each; those inside 2h (:218) are packed into the buffer and their terms
-  // summed 32 at a time.  KEEP (first pass): the candidates within 2 h_high
-  // are recorded, in order, in j's row of `prune`.
-  auto dscan = [&](int j, int nc, auto getq, auto u_, auto keep_, int& kept, double& part) {
-    constexpr int U = decltype(u_)::value;
-    constexpr bool KEEP = decltype(keep_)::value;
-    const double xj = W.x[j], yj = W.y[j], zj = W.z[j], hsj = W.hs[j];
-    const int pj = W.p[j];
-    int nin = 0;
-    for (int b = 0; b < nc; b += 32 * U) {
-      int q[U];
-      double4 Q[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int k = b + 32 * u + lane;
-        q[u] = k < nc ? getq(k) : pj;
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) Q[u] = pm[q[u]];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const double d0 = Q[u].x - xj, d1 = Q[u].y - yj, d2 = Q[u].z - zj;
-        const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
-        const bool in = q[u] != pj && drsqd < hsj;
-        const unsigned mi = __ballot_sync(FULL, in);
-        if (in) {
-          const int o = nin + __popc(mi & lt);
-          W.d2[o] = drsqd;
-          W.m[o] = Q[u].w;
-        }
-        nin += __popc(mi);
-        if constexpr (KEEP) {
-          const bool keep = q[u] != pj && drsqd < W.hh[j];
-          const unsigned mk = __ballot_sync(FULL, keep);
-          const int pos = kept + __popc(mk & lt);
-          if (keep && pos < L) prune[(size_t)pj * L + pos] = q[u];
-          kept += __popc(mk);
-        }
-      }
-      if (nin > GP_PINB - 32 * U || b + 32 * U >= nc) {
-        __syncwarp();
-        const double ihj = W.ih[j], hfj = W.hf[j];
-        for (int t = lane; t < nin; t += 32) gh_density_in(W.d2[t], W.m[t], ihj, hfj, part);
-        nin = 0;
-        __syncwarp();
-      }
-    }
-    niter += (nc + 31) >> 5;
-  };
-
-  // Final-pass sums (:360-425) of particle j over the candidates getq(0..nc),
-  // its velocity vj
-  auto fscan = [&](int j, int nc, auto getq, auto u_, double vxj, double vyj, double vzj,
-                   GhFinal& part, int& gcnt) {
-    constexpr int U = decltype(u_)::value;
-    const double xj = W.x[j], yj = W.y[j], zj = W.z[j], hsj = W.hs[j];
-    const int pj = W.p[j];
-    int nin = 0;
-    for (int b = 0; b < nc; b += 32 * U) {
-      int q[U];
-      double4 Q[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int k = b + 32 * u + lane;
-        q[u] = k < nc ? getq(k) : pj;
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) Q[u] = pm[q[u]];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const double d0 = Q[u].x - xj, d1 = Q[u].y - yj, d2 = Q[u].z - zj;
-        const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
-        const bool in = q[u] != pj && drsqd <= hsj;                   // :360
-        const unsigned mi = __ballot_sync(FULL, in);
-        if (in) {
-          const double4 V = vel[q[u]];
-          const double dv0 = V.x - vxj, dv1 = V.y - vyj, dv2 = V.z - vzj;
-          const int o = nin + __popc(mi & lt);
-          W.d2[o] = drsqd;
-          W.m[o] = Q[u].w;
-          W.dv[o] = (dv0 * d0 + dv1 * d1) + dv2 * d2;
-          // the gather neighbours r^2 <= 4h^2 of the neighbour lists, in
-          // order, into the particle's own row of prune: each goes to a slot
-          // at or before the candidate it came from, whose read is done (the
-          // ballot above waits for every lane's candidate), so no candidate
-          // still to be read is overwritten
-          if (rec && gcnt + o < L) prune[(size_t)pj * L + gcnt + o] = q[u];
-        }
-        nin += __popc(mi);
-      }
-      if (nin > GP_PINB - 32 * U || b + 32 * U >= nc) {
-        __syncwarp();
-        gcnt += nin;
-        const double ihj = W.ih[j], hfj = W.hf[j];
-        for (int t = lane; t < nin; t += 32)
-          gh_final_in(W.d2[t], W.m[t], W.dv[t], ihj, hfj, part);
-        nin = 0;
-        __syncwarp();
-      }
-    }
-    niter += (nc + 31) >> 5;
-  };
-
-  for (int g = gr_next(work, lane); (long long)g * 32 < nact; g = gr_next(work, lane)) {
-    const int i = g * 32 + lane;
-    bool live;
-    const int p = group_particle(i, nact, act, live);
+  for (int g = gr_next(work, lane); (long long)g << lpw < nact; g = gr_next(work, lane)) {
+    const int i = (g << lpw) + lane;
+    int p = lane < PW && i < nact ? (act ? act[i] : i) : -1;
+    const bool live = p >= 0;
+    const int p0 = __shfl_sync(FULL, p, 0);
+    if (p0 < 0) continue;                              // a group of padding only
+    p = live ? p : p0;
     const double rextent = cl ? cl[cloud_of(cl, ncl, p)].rextent : rextent0;
-    const int n = live ? nleaf[p] : 0;
+    const int n = live ? nrow[p] : 0;
     const double4 P = pm[p];
     const double mp = P.w;
     GhState s;
@@ -715,52 +782,70 @@ __global__ void __launch_bounds__(GP_THREADS, 8) k_gradh_pass(
     W.x[lane] = P.x;
     W.y[lane] = P.y;
     W.z[lane] = P.z;
-    // The candidates within 2 h_high of the particle, recorded in its row of
-    // `prune` by the first pass: every later pass has h <= h_high (else the
-    // particle walks again), so they hold all the candidates it can count.
-    W.hh[lane] = (KERNRANGESQD * s.h_high) * s.h_high;
     W.p[lane] = p;
     W.n[lane] = n;
-    W.npr[lane] = -1;
-    bool first = true;
-    double rt = 0.0;
+    const double wself = (mp * tabA[0].x);
     while (true) {
       const unsigned A = __ballot_sync(FULL, active);
       if (A == 0u) break;
       const double ih = 1.0 / s.hp;                                    // :199-235
       const double hf = pow(ih, NDIMPR);
       W.ih[lane] = ih;
-      W.hf[lane] = hf;
       W.hs[lane] = (KERNRANGESQD * s.hp) * s.hp;
+      if (active) W.list[__popc(A & lt)] = lane;
+      const int na = __popc(A);
       __syncwarp();
-      for (unsigned todo = A; todo != 0u; todo &= todo - 1u) {
-        const int j = __ffs(todo) - 1;
-        double part = 0.0;
-        int kept = 0;
-        const int nprj = W.npr[j];
-        if (first || nprj < 0) {
-          const int nj = W.n[j];
-          const int* row = leaves + (size_t)W.p[j] * GH_LEAVES;
-          for (int s0 = 0; s0 < nj; s0 += GP_PSEG) {   // the row, GP_PSEG leaves at a time
-            const int nc = gp_flatten(row + s0, min(GP_PSEG, nj - s0), W.cand, lane);
-            auto fromrow = [&](int k) { return W.cand[k]; };
-            if (first) dscan(j, nc, fromrow, ICst<2>{}, std::true_type{}, kept, part);
-            else dscan(j, nc, fromrow, ICst<2>{}, std::false_type{}, kept, part);
+      for (int r0 = 0; r0 < na; r0 += 4) {
+        const bool has = r0 + quad < na;
+        const int j = W.list[has ? r0 + quad : r0];
+        const int nj = has ? W.n[j] : 0;
+        const int pj = W.p[j];
+        const int* row = rows + (size_t)pj * GH_LEAVES;
+        const double xj = W.x[j], yj = W.y[j], zj = W.z[j], ihj = W.ih[j];
+        const double ih2 = ihj * ihj;
+        double sum = 0.0;
+        int nmax = max(nj, __shfl_xor_sync(FULL, nj, 8));
+        nmax = max(nmax, __shfl_xor_sync(FULL, nmax, 16));
+        for (int k = l8; k - l8 < nmax; k += 8 * U) {
+          int q[U], kern[U];
+          double4 Q[U];
+          gp_load<U>(row, k, nj, pj, pm, q, Q);
+          double d2[U];
+          unsigned bad = 0u;
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const double d0 = Q[u].x - xj, d1 = Q[u].y - yj, dz = Q[u].z - zj;
+            d2[u] = fma(dz, dz, fma(d1, d1, d0 * d0));
+            bool sure;
+            kern[u] = gh_bin(d2[u] * ih2, sure);
+            if (q[u] == pj) Q[u].w = 0.0;                              // not the particle itself
+            else if (!sure) bad |= 1u << u;
           }
-          if (first && lane == 0) W.npr[j] = kept <= L ? kept : -1;
-        } else {
-          const int* prj = prune + (size_t)W.p[j] * L;
-          dscan(j, nprj, [&](int k) { return prj[k]; }, ICst<4>{}, std::false_type{}, kept,
-                part);
+          if (__any_sync(FULL, bad != 0u)) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if ((bad >> u) & 1u) kern[u] = gh_bin_exact(d2[u], ihj);
+          }
+          // (beyond 2h, :218, the kernel is zero)
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            double a, b;
+            gh_uv(kern[u], a, b);
+            sum = fma(Q[u].w, fma(-4.0 * b, b * b, a * (a * a)), sum);
+          }
         }
-        const double sum = warp_sum(part);
-        if (lane == j) rt = sum;
+        __syncwarp();
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
+        if (l8 == 0 && has) W.part[j][0] = sum;
+        niter += (nj + 31) >> 5;
       }
-      first = false;
+      __syncwarp();
       if (active) {
         ++npass;
         ncands += s.pp_pot;
-        if (gh_after_pass(s, mp, h_fac, rextent, (mp * tabA[0].x) * hf + rt)) active = false;
+        const double rt = fma(hf * (0.25e-12 * INVPI), W.part[lane][0], wself * hf);
+        if (gh_after_pass(s, mp, h_fac, rextent, rt)) active = false;
         else if (s.hp > s.h_high) {                                    // :154-170 would walk again
           single = true;
           active = false;
@@ -768,67 +853,92 @@ __global__ void __launch_bounds__(GP_THREADS, 8) k_gradh_pass(
       }
       __syncwarp();
     }
-    // final pass (:317-425)
+    // final pass (:317-425), from candidates that hold every particle within 2h
+    // while h < h_high
+    const double hp = h_fac * pow(mp / s.rho, ONETHIRD);
+    if (live && !single && !(hp < s.h_high)) single = true;
     const bool ok = live && !single;
     const unsigned F = __ballot_sync(FULL, ok);
-    const double hp = h_fac * pow(mp / s.rho, ONETHIRD);
     const double ih = 1.0 / hp;
     const double hf = pow(ih, NDIMPR);
-    const double4 vp = vel[p];
     W.ih[lane] = ih;
-    W.hf[lane] = hf;
     W.hs[lane] = (KERNRANGESQD * hp) * hp;
-    // the recorded candidates serve when 2h < 2 h_high (those within 2h of the
-    // final h are among them)
-    if (!(hp < s.h_high)) W.npr[lane] = -1;
-    const unsigned cplm = __ballot_sync(FULL, hp < s.h_high);
+    if (ok) W.list[__popc(F & lt)] = lane;
+    const int nf = __popc(F);
     __syncwarp();
-    GhFinal f;
-    gh_final_init(f, mp, ih, hf, tabA[0]);
-    for (unsigned todo = F; todo != 0u; todo &= todo - 1u) {
-      const int j = __ffs(todo) - 1;
-      const double vxj = __shfl_sync(FULL, vp.x, j), vyj = __shfl_sync(FULL, vp.y, j),
-                   vzj = __shfl_sync(FULL, vp.z, j);
-      const int nprj = W.npr[j];
-      GhFinal part;
-      part.rt = 0.0; part.om = 0.0; part.dv = 0.0; part.zt = 0.0;
+    for (int r0 = 0; r0 < nf; r0 += 4) {
+      const bool has = r0 + quad < nf;
+      const int j = W.list[has ? r0 + quad : r0];
+      const int nj = has ? W.n[j] : 0;
+      const int pj = W.p[j];
+      const int* row = rows + (size_t)pj * GH_LEAVES;
+      int* grow = gset + (size_t)pj * L;
+      const double xj = W.x[j], yj = W.y[j], zj = W.z[j], hsj = W.hs[j], ihj = W.ih[j];
+      const double ih2 = ihj * ihj;
+      const double4 vj = vel[pj];
+      double srt = 0.0, som = 0.0, sdv = 0.0, szt = 0.0;
       int gcnt = 0;
-      if (nprj < 0) {
-        const int nj = W.n[j];
-        const int* row = leaves + (size_t)W.p[j] * GH_LEAVES;
-        for (int s0 = 0; s0 < nj; s0 += GP_PSEG) {     // the row, GP_PSEG leaves at a time
-          const int nc = gp_flatten(row + s0, min(GP_PSEG, nj - s0), W.cand, lane);
-          fscan(j, nc, [&](int k) { return W.cand[k]; }, ICst<1>{}, vxj, vyj, vzj, part, gcnt);
+      int nmax = max(nj, __shfl_xor_sync(FULL, nj, 8));
+      nmax = max(nmax, __shfl_xor_sync(FULL, nmax, 16));
+      for (int k = l8; k - l8 < nmax; k += 8 * UF) {
+        int q[UF];
+        double4 Q[UF];
+        gp_load<UF>(row, k, nj, pj, pm, q, Q);
+#pragma unroll
+        for (int u = 0; u < UF; ++u) {
+          const double d0 = Q[u].x - xj, d1 = Q[u].y - yj, d2 = Q[u].z - zj;
+          const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
+          const bool in = q[u] != pj && drsqd <= hsj;                  // :360
+          if (rec) {                                   // the gather neighbours, in order
+            const unsigned bg = (__ballot_sync(FULL, in) >> (lane & 24)) & 0xffu;
+            const int o = gcnt + __popc(bg & ((1u << l8) - 1u));
+            if (in && o < L) grow[o] = q[u];
+            gcnt += __popc(bg);
+          }
+          const double4 V = vel[in ? q[u] : pj];
+          bool sure;
+          int kern = gh_bin(drsqd * ih2, sure);
+          if (__any_sync(FULL, in && !sure)) {
+            if (in && !sure) kern = gh_bin_exact(drsqd, ihj);
+          }
+          double a, b;
+          gh_uv(kern, a, b);
+          const double s4 = int_double(2 * kern + 1);
+          const double u2 = a * a, v2 = b * b;
+          const double a2 = fma(-4.0, v2, u2);                         // 1e8 w4 / (-3/4)
+          const double a3 = fma(-4.0 * b, v2, a * u2);                 // 1e12 w0 / (1/4)
+          const double m = in ? Q[u].w : 0.0;
+          const double dvdr = fma(V.z - vj.z, d2, fma(V.y - vj.y, d1, (V.x - vj.x) * d0));
+          srt = fma(m, a3, srt);
+          som = fma(m, fma(s4, a2, -a3), som);
+          sdv = fma(m * dvdr, a2 * rsqrt(drsqd + 1.0e-200), sdv);
+          szt = fma(m, fma(u2 * u2, fma(-0.2e-4, a, 0.5), -(v2 * v2) * fma(-0.8e-4, b, 1.0)), szt);
         }
-      } else {
-        const int* prj = prune + (size_t)W.p[j] * L;
-        fscan(j, nprj, [&](int k) { return prj[k]; }, ICst<2>{}, vxj, vyj, vzj, part, gcnt);
       }
-      // the gather count (the row's first entries; pptot grows with the
-      // scatter neighbours later), or -1 when the candidates may miss some
-      // particle within 2h (h >= h_high: the neighbour walk completes the row)
-      if (rec && lane == 0) {
-        const int pj = W.p[j];
-        if ((cplm >> j) & 1u) {
-          npot[pj] = gcnt;
-          pptot[pj] = gcnt;
-        } else {
-          npot[pj] = -1;
-        }
-      }
-      const double srt = warp_sum(part.rt), som = warp_sum(part.om), sdv = warp_sum(part.dv),
-                   szt = warp_sum(part.zt);
-      if (lane == j) {
-        f.rt = f.rt + srt;
-        f.om = f.om + som;
-        f.dv = f.dv + sdv;
-        f.zt = f.zt + szt;
-      }
+      __syncwarp();
+      const double v = sum4_by8(srt, som, sdv, szt, lane);
+      if (has && (lane & 1) == 0) W.part[j][l8 >> 1] = v;
+      if (has && l8 == 0) W.g[j] = gcnt;
+      niter += (nj + 31) >> 5;
     }
+    __syncwarp();
     if (ok) {
       ++npass;
       ncands += s.pp_pot;
+      const double q = 0.25 * INVPI;
+      GhFinal f;
+      gh_final_init(f, mp, ih, hf, tabA[0]);
+      f.rt = fma(1.0e-12 * q * hf, W.part[lane][0], f.rt);
+      f.om = fma(3.0e-12 * q * (hf * ih), W.part[lane][1], f.om);      // wh = 3/4 (s a2 - a3)
+      f.dv = fma(3.0e-8 * q * (hf * ih), W.part[lane][2], f.dv);       // -w4 = 3/4 a2
+      f.zt = fma(1.0e-16 * (ih * ih), W.part[lane][3], f.zt);
       gh_store(p, mp, hp, f, hz, rho, omega, divv, drhodt, err);
+      // the gather count (the row's first entries; pptot grows with the
+      // scatter neighbours later)
+      if (rec) {
+        npot[p] = W.g[lane];
+        pptot[p] = W.g[lane];
+      }
     }
     if (single) {
       ++nsingle;
@@ -836,10 +946,10 @@ __global__ void __launch_bounds__(GP_THREADS, 8) k_gradh_pass(
       if (rec) npot[p] = -1;                       // its neighbour list: from a walk
     }
   }
-  atomicAdd(counts + 5, (unsigned long long)npass);
-  atomicAdd(counts + 6, (unsigned long long)ncands);
-  atomicAdd(counts + 15, (unsigned long long)nsingle);
-  if (lane == 0) atomicAdd(counts + 13, (unsigned long long)niter);
+  warp_count(counts + 5, npass, lane);
+  warp_count(counts + 6, ncands, lane);
+  warp_count(counts + 15, nsingle, lane);
+  warp_count(counts + 13, niter, lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -1785,7 +1895,8 @@ __global__ void __launch_bounds__(GP_THREADS) k_neib_rows(
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int* cand = cand_all[w];
   const unsigned lt = (1u << lane) - 1u;
-  unsigned long long ncands = 0, niter = 0, nsingle = 0;
+  unsigned long long ncands = 0, niter = 0;
+  unsigned nsingle = 0;
   for (int g = gr_next(work, lane); (long long)g * 32 < nact; g = gr_next(work, lane)) {
     const int i = g * 32 + lane;
     bool live;
@@ -1834,7 +1945,7 @@ __global__ void __launch_bounds__(GP_THREADS) k_neib_rows(
     }
     __syncwarp();
   }
-  atomicAdd(counts + 15, nsingle);
+  warp_count(counts + 15, nsingle, lane);
   if (lane == 0) {
     atomicAdd(counts + 7, ncands);
     atomicAdd(counts + 14, niter);
@@ -2102,6 +2213,7 @@ HydroTree hydro_tree(const Ctx& c) {
 }  // namespace
 
 constexpr size_t GR_SMEM = sizeof(GrShared) * GR_WARPS;
+constexpr size_t GH_SMEM = sizeof(GhShared) * GR_WARPS;
 
 // Resident blocks per SM of the group-walk kernels on device dev (their
 // dynamic shared-memory limit is raised on first use per device).
@@ -2112,8 +2224,8 @@ static int gr_blocks_per_sm(int dev, int which) {
   int& r = o[which];
   if (r == 0) {
     if (which == 0) {
-      cudaFuncSetAttribute(k_gradh_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GR_SMEM);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_gradh_walk, GR_THREADS, GR_SMEM);
+      cudaFuncSetAttribute(k_gradh_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GH_SMEM);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_gradh_walk, GR_THREADS, GH_SMEM);
     } else {
       cudaFuncSetAttribute(k_neib_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GR_SMEM);
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_neib_walk, GR_THREADS, GR_SMEM);
@@ -2164,12 +2276,16 @@ void launch_gradh(Ctx& c, int nact) {
   // with every particle active, the final passes record each particle's
   // gather neighbours for the neighbour lists that follow (launch_neib)
   const bool rec = c.act == nullptr;
+  // the groups of the walk: as wide as the gravity walk's (grav_lpw)
   int ngrp = nact;
   const int* gl = group_list(c, ngrp);
+  const bool forest = gl != c.act;
+  const int wlpw = grav_lpw(nact);
+  const int nwg = forest ? c.nggrp : nb(nact, 1 << wlpw);
   cudaMemsetAsync(c.work, 0, sizeof(int), c.st);
-  k_gradh_walk<<<gr_grid(c, ngrp, 0), GR_THREADS, GR_SMEM, c.st>>>(
-      ngrp, gl, c.pm, c.hz, t, c.leaves, c.nleaf, c.npot, c.wstack, c.wstack_cap, counts,
-      c.work);
+  k_gradh_walk<<<gr_grid(c, nwg * 32, 0), GR_THREADS, GH_SMEM, c.st>>>(
+      ngrp, gl, nwg, forest ? c.ggrp : nullptr, wlpw, c.pm, c.hz, t, c.leaves, c.nleaf, c.npot,
+      c.wstack, c.wstack_cap, counts, c.work);
   finish_reorder(c);            // velocities still arriving: the passes need them from here on
   static int occ[16] = {};
   int& o = occ[c.dev >= 0 && c.dev < 16 ? c.dev : 0];
@@ -2178,10 +2294,13 @@ void launch_gradh(Ctx& c, int nact) {
     if (o < 1) o = 1;
   }
   const int bps = c.tune.gradh_bps > 0 ? std::min(o, c.tune.gradh_bps) : o;
-  const int blocks = std::min(sm_count(c) * bps, nb(nb(ngrp, 32), GP_WARPS));
+  // particles per warp: 32, or fewer down to 4 so that every resident warp gets some
+  int lpw = 5;
+  while (lpw > 2 && nb(ngrp, 1 << lpw) < 2 * sm_count(c) * bps * GP_WARPS) --lpw;
+  const int blocks = std::min(sm_count(c) * bps, nb(nb(ngrp, 1 << lpw), GP_WARPS));
   cudaMemsetAsync(c.work, 0, 3 * sizeof(int), c.st);     // group counter, nredo, nwide
   k_gradh_pass<<<blocks, GP_THREADS, 0, c.st>>>(
-      ngrp, gl, c.pm, c.hz, c.vel, c.rho, c.omega, c.div_v, c.drhodt, c.tabA, c.prm.h_fac,
+      ngrp, gl, lpw, c.pm, c.hz, c.vel, c.rho, c.omega, c.div_v, c.drhodt, c.tabA, c.prm.h_fac,
       c.prm.pp_gather, c.info.rextent, c.leaves, c.nleaf, c.npot, c.redo, c.work + 1,
       c.pplist, c.prm.pp_limit, c.d_err, counts, c.work, t.cl, t.ncl, rec ? 1 : 0, c.pptot);
   // three walk-stack slots of scratch per redo warp

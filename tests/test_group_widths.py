@@ -31,8 +31,10 @@ def test_gravity_at_the_width_edges(n):
             # sums of about 1000 terms of a few 2^-52 each
             assert rel_rows(ag, ao).max() < 1e-11 and rel_rows(pg, po).max() < 1e-12
         else:
-            # 32-bit terms: a few 2^-24 of the largest contributions
-            assert rel_scaled(ag, ao) < 1e-5 and rel_rows(pg, po).max() < 1e-6
+            # 32-bit terms: a few 2^-24 of the largest contributions, and a pair that the
+            # 32-bit separation puts into the next bin of the kernel (2e-4 h wide)
+            # changes its term by up to 1e-4, of a sum of at least 32
+            assert rel_scaled(ag, ao) < 1e-5 and rel_rows(pg, po).max() < 1e-5
     o.close()
 
 
