@@ -259,8 +259,7 @@ void free_all(Ctx& c) {
                 c.drhodt_alt, c.press, c.sound, c.acc, c.gpot,
                 c.pf, c.hf4,
                 c.pptot, c.pplist, c.stage, c.istage, c.keys, c.keys_alt, c.keys_hi, c.keys_lo, c.idx, c.idx_alt,
-                c.rs_hist, c.bbox_part, c.branch, c.branch_next, c.nchild, c.choff, c.cstart,
-                c.bflag, c.bscan, c.leaf, c.nextcell, c.ifopen, c.pstart, c.pcount, c.parent,
+                c.rs_hist, c.bbox_part, c.blk_count, c.bflag, c.bscan, c.pcount, c.parent,
                 c.level, c.nkids, c.work, c.sinks, c.wstack, c.leaves, c.nleaf, c.npot, c.redo, c.wide, c.wst, c.wacc, c.link, c.gA, c.gB, c.gC, c.wA, c.hN, c.hA, c.hrm, c.hA32, c.hrm32, c.hmax, c.bbmin, c.bbmax, c.d_info,
                 c.d_err, c.d_counts, c.sink_out, c.tabA, c.tabG, c.scan.total, c.scan.level_buf[0],
                 c.scan.level_buf[1], c.scan.level_buf[2], c.scan.level_buf[3]};
@@ -289,8 +288,7 @@ int alloc_all(Ctx& c) {
   const size_t P = (size_t)c.pmax;
   const size_t C = (size_t)c.cmax + 1;
   const size_t L = (size_t)c.prm.pp_limit;
-  const size_t nbr = P / 9 + 2;
-  const size_t rsblk = (P + 4095) / 4096;
+  const size_t rsh = radix_hist_ints(P);
   int bad = 0;
   bad |= alloc(c.pm, P) | alloc(c.hz, P) | alloc(c.vel, P) | alloc(c.csq, P) | alloc(c.orig, P);
   bad |= alloc(c.pm_alt, P) | alloc(c.hz_alt, P) | alloc(c.vel_alt, P) | alloc(c.csq_alt, P) |
@@ -305,11 +303,9 @@ int alloc_all(Ctx& c) {
          alloc(c.istage, P * L + P);
   bad |= alloc(c.keys, P) | alloc(c.keys_alt, P) | alloc(c.keys_hi, P) | alloc(c.keys_lo, P) |
          alloc(c.idx, P) | alloc(c.idx_alt, P) |
-         alloc(c.rs_hist, 256 * rsblk) | alloc(c.bbox_part, 6 * 1184);
-  bad |= alloc(c.branch, nbr) | alloc(c.branch_next, nbr) | alloc(c.nchild, nbr) |
-         alloc(c.choff, nbr) | alloc(c.cstart, 9 * nbr) | alloc(c.bflag, C) | alloc(c.bscan, C);
-  bad |= alloc(c.leaf, C) | alloc(c.nextcell, C) | alloc(c.ifopen, C) | alloc(c.pstart, C) |
-         alloc(c.pcount, C) | alloc(c.parent, C) | alloc(c.level, C) | alloc(c.link, C);
+         alloc(c.rs_hist, rsh) | alloc(c.bbox_part, 6 * 1184) |
+         alloc(c.blk_count, 32 * ((P + 255) / 256)) | alloc(c.bflag, C) | alloc(c.bscan, C);
+  bad |= alloc(c.pcount, C) | alloc(c.parent, C) | alloc(c.level, C) | alloc(c.link, C);
   bad |= alloc(c.hA32, C) | alloc(c.hrm32, C) | alloc(c.nkids, C) | alloc(c.work, 4);
   bad |= alloc(c.leaves, P * 256) | alloc(c.nleaf, P) | alloc(c.npot, P) | alloc(c.redo, P) | alloc(c.wide, P);
   bad |= wide_scratch_alloc(c);
@@ -323,7 +319,7 @@ int alloc_all(Ctx& c) {
   c.wstack_cap = grav_walk_stack_cap(c);
   bad |= alloc(c.wstack, (size_t)c.wstack_slots * c.wstack_cap);
   if (bad) return -1;
-  const size_t scan_n = std::max(std::max(256 * rsblk, C), P) + 16;
+  const size_t scan_n = std::max(std::max(rsh, C), P) + 16;
   if (scan_scratch_alloc(c.scan, (int)scan_n)) return -1;
   cudaMemset(c.d_err, 0, sizeof(DevError));
   cudaMemset(c.d_counts, 0, sizeof(int) * 32);

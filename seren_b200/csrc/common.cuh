@@ -74,13 +74,12 @@ __device__ __forceinline__ void set_error(DevError* e, int code, int where, int 
 struct TreeInfo {
   int ctot;          // last cell id
   int ltot;          // deepest level
-  int nbranch;       // branch cells on the level being split
-  int nchild;        // children made on that level
   double rextent;    // maxval(rmax - rmin) of the bounding box (bounding_box.F90:348)
   double root[3];    // root cell centre
   double cellsize;   // 0.5*maxval(rmax - rmin) (BHgrav_build.F90:66)
   int first_cell[32];
   int last_cell[32];
+  int ncell[32];     // cells per level
 };
 
 // One of several independent clouds sharing a context (seren_gpu_set_clouds).

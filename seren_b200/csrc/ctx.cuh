@@ -123,20 +123,13 @@ struct Ctx {
   int* idx_alt = nullptr;
   int* rs_hist = nullptr;     // [256][nblk]
   double* bbox_part = nullptr;
-  int* branch = nullptr;      // branch cells of the level being split
-  int* branch_next = nullptr;
-  int* nchild = nullptr;      // children per branch cell
-  int* choff = nullptr;       // exclusive scan of nchild
-  int* cstart = nullptr;      // [nbranch][9] child range boundaries
-  int* bflag = nullptr;       // 1 for a branch child on the new level
+  int* blk_count = nullptr;   // [32][blocks] cell starts per level and block of particles
+  bool deep_sort = false;     // the last tree had more levels than the short sort orders
+  int* bflag = nullptr;       // flags and their scan (lists of particles and cells)
   int* bscan = nullptr;
   ScanScratch scan;
 
   // tree, breadth-first cell ids 0..ctot
-  int* leaf = nullptr;
-  int* nextcell = nullptr;
-  int* ifopen = nullptr;
-  int* pstart = nullptr;
   int* pcount = nullptr;
   int* parent = nullptr;
   int* level = nullptr;
@@ -264,6 +257,7 @@ void launch_update_hmax(Ctx& c);      // BHhydro_update_hmax
 void launch_hguess(Ctx& c);           // BHhydro_hguess
 void scan_exclusive(Ctx& c, const int* in, int* out, int n);   // total -> c.scan.total
 int scan_scratch_alloc(ScanScratch& s, int nmax);
+size_t radix_hist_ints(size_t pmax);  // c.rs_hist of a sort of up to pmax items
 
 // blockstep.cu
 void reorder_block(Ctx& c);           // the block state follows a build's permutation

@@ -9,8 +9,9 @@
 // sort: each particle's octant path is computed from the same FP64 centre
 // comparisons (rp > rc with rc built by repeated +/- cellsize), packed into a
 // 63-bit key, and stably radix-sorted; cells are then the runs of a common
-// prefix, emitted level by level in breadth-first order, and each leaf's
-// particles are put back into input-index order.
+// prefix, numbered breadth-first from per-level counts and written for all
+// levels at once, and each leaf's particles are put back into input-index order.
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 
@@ -132,15 +133,16 @@ __global__ void k_bbox_final(const double* __restrict__ part, int nblk, TreeInfo
   for (int k = 0; k < 3; ++k) info->root[k] = 0.5 * (rmin[k] + rmax[k]);
 }
 
-// the same per cloud of a forest, one block per cloud; cloud 0 also fills the
-// tree summary's root box
-__global__ void k_bbox_clouds(const double4* __restrict__ pm, CloudInfo* cl, TreeInfo* info) {
+// the same per cloud of a forest, gridDim.y blocks per cloud: block (k, s) the
+// extremes of slice s of cloud k, then (k_bbox_clouds) the cloud's root box from
+// its slices; cloud 0 also fills the tree summary's root box
+__global__ void k_bbox_cloud_part(const double4* __restrict__ pm,
+                                  const CloudInfo* __restrict__ cl, double* __restrict__ part) {
   __shared__ double s[6][BB_T];
-  CloudInfo& C = cl[blockIdx.x];
-  const int p0 = C.pstart, n = C.n;
+  const int p0 = cl[blockIdx.x].pstart, n = cl[blockIdx.x].n;
   double mx[3] = {-BIG_NUMBER, -BIG_NUMBER, -BIG_NUMBER};
   double mn[3] = {BIG_NUMBER, BIG_NUMBER, BIG_NUMBER};
-  for (int i = threadIdx.x; i < n; i += BB_T) {
+  for (int i = blockIdx.y * BB_T + threadIdx.x; i < n; i += gridDim.y * BB_T) {
     const double4 p = pm[p0 + i];
     mx[0] = fmax(mx[0], p.x); mx[1] = fmax(mx[1], p.y); mx[2] = fmax(mx[2], p.z);
     mn[0] = fmin(mn[0], p.x); mn[1] = fmin(mn[1], p.y); mn[2] = fmin(mn[2], p.z);
@@ -155,19 +157,34 @@ __global__ void k_bbox_clouds(const double4* __restrict__ pm, CloudInfo* cl, Tre
       }
     __syncthreads();
   }
-  if (threadIdx.x != 0) return;
-  const double rmax[3] = {s[0][0], s[1][0], s[2][0]};
-  const double rmin[3] = {s[3][0], s[4][0], s[5][0]};
-  const double ext = fmax(fmax(rmax[0] - rmin[0], rmax[1] - rmin[1]), rmax[2] - rmin[2]);
+  if (threadIdx.x < 6)
+    part[((size_t)blockIdx.x * gridDim.y + blockIdx.y) * 6 + threadIdx.x] = s[threadIdx.x][0];
+}
+
+__global__ void k_bbox_clouds(int ncl, int nslice, const double* __restrict__ part, CloudInfo* cl,
+                              TreeInfo* info) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= ncl) return;
+  CloudInfo& C = cl[k];
+  double mx[3] = {-BIG_NUMBER, -BIG_NUMBER, -BIG_NUMBER};
+  double mn[3] = {BIG_NUMBER, BIG_NUMBER, BIG_NUMBER};
+  for (int b = 0; b < nslice; ++b) {
+    const double* p = part + ((size_t)k * nslice + b) * 6;
+    for (int d = 0; d < 3; ++d) {
+      mx[d] = fmax(mx[d], p[d]);
+      mn[d] = fmin(mn[d], p[3 + d]);
+    }
+  }
+  const double ext = fmax(fmax(mx[0] - mn[0], mx[1] - mn[1]), mx[2] - mn[2]);
   C.rextent = ext;
   C.cellsize = 0.5 * ext;
-  for (int k = 0; k < 3; ++k) C.root[k] = 0.5 * (rmin[k] + rmax[k]);
+  for (int d = 0; d < 3; ++d) C.root[d] = 0.5 * (mn[d] + mx[d]);
   C.delta = (float)(ldexp(1.0, -22) * (C.cellsize > 0.0 ? C.cellsize : 1.0));
-  C.cell = blockIdx.x;
-  if (blockIdx.x == 0) {
+  C.cell = k;
+  if (k == 0) {
     info->rextent = C.rextent;
     info->cellsize = C.cellsize;
-    for (int k = 0; k < 3; ++k) info->root[k] = C.root[k];
+    for (int d = 0; d < 3; ++d) info->root[d] = C.root[d];
   }
 }
 
@@ -262,13 +279,16 @@ __global__ void k_gather_hi(const unsigned long long* __restrict__ hi, const int
 // stable LSD radix sort of (64-bit key, int) pairs, 8-bit digits
 constexpr int RS_T = 256;
 constexpr int RS_W = RS_T / 32;
-constexpr int RS_I = 16;                  // items per lane
-constexpr int RS_TILE = RS_T * RS_I;      // 4096 items per block
-constexpr int RS_CHUNK = 32 * RS_I;       // 512 contiguous items per warp
+// Items per lane: 16 (tiles of 4096), or 4 below RS_SMALL items, where tiles of
+// 4096 leave most SMs without one (a scatter pass of 32768 items: 16.5 us on 8
+// tiles, 7 us on 32).
+constexpr int RS_SMALL = 1 << 19;
 
+template <int RS_I>
 __global__ void k_rs_hist(const unsigned long long* __restrict__ keys, int n, int shift,
                           int* __restrict__ hist, int nblk) {
   __shared__ int cnt[256];
+  constexpr int RS_TILE = RS_T * RS_I;
   cnt[threadIdx.x] = 0;
   __syncthreads();
   const long base = (long)blockIdx.x * RS_TILE;
@@ -286,15 +306,19 @@ __global__ void k_rs_hist(const unsigned long long* __restrict__ keys, int n, in
 // consecutive threads write consecutive slots of a digit's run, so the stores
 // coalesce.  Shared memory: the tile's keys and values, the per-warp digit
 // counts and the tile's digit starts.
-constexpr size_t RS_SMEM = (size_t)RS_TILE * (sizeof(unsigned long long) + sizeof(int)) +
-                           sizeof(int) * (RS_W * 256 + 256 + RS_W);
+constexpr size_t rs_smem(int items) {
+  return (size_t)RS_T * items * (sizeof(unsigned long long) + sizeof(int)) +
+         sizeof(int) * (RS_W * 256 + 256 + RS_W);
+}
+template <int RS_I>
 __global__ void __launch_bounds__(RS_T) k_rs_scatter(const unsigned long long* __restrict__ kin,
                                                      const int* __restrict__ vin,
                                                      unsigned long long* __restrict__ kout,
                                                      int* __restrict__ vout, int n, int shift,
                                                      const int* __restrict__ offs, int nblk) {
-  extern __shared__ __align__(16) unsigned char rs_smem[];
-  unsigned long long* sk = reinterpret_cast<unsigned long long*>(rs_smem);
+  constexpr int RS_TILE = RS_T * RS_I, RS_CHUNK = 32 * RS_I;   // a warp's items are contiguous
+  extern __shared__ __align__(16) unsigned char rs_buf[];
+  unsigned long long* sk = reinterpret_cast<unsigned long long*>(rs_buf);
   int* sv = reinterpret_cast<int*>(sk + RS_TILE);
   int (*wh)[256] = reinterpret_cast<int (*)[256]>(sv + RS_TILE);
   int* tstart = reinterpret_cast<int*>(wh + RS_W);
@@ -363,165 +387,295 @@ __global__ void __launch_bounds__(RS_T) k_rs_scatter(const unsigned long long* _
   }
 }
 
-// ---------------------------------------------------------------------------
-// breadth-first cell emission
-__global__ void k_root(int n, int cmax, int* leaf, int* nextcell, int* ifopen, int* pstart,
-                       int* pcount, int* parent, int* level, int* branch, TreeInfo* info) {
-  leaf[0] = 0;                 // the root is always split (BHgrav_build.F90:74)
-  nextcell[0] = cmax + 1;      // :75
-  ifopen[0] = -1;
-  pstart[0] = 0;
-  pcount[0] = n;
-  parent[0] = -1;
-  level[0] = 0;
-  branch[0] = 0;
-  info->nbranch = 1;
-  info->ctot = 0;
-  info->first_cell[0] = 0;
-  info->last_cell[0] = 0;
-}
-
-// the roots of a forest: cell k is cloud k's root (always split, as the
-// single root, BHgrav_build.F90:74-75), its particles the cloud's sorted range
-__global__ void k_roots(int ncl, const CloudInfo* __restrict__ cl, int cmax, int* leaf,
-                        int* nextcell, int* ifopen, int* pstart, int* pcount, int* parent,
-                        int* level, int* branch, TreeInfo* info) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < ncl) {
-    leaf[k] = 0;
-    nextcell[k] = cmax + 1;
-    ifopen[k] = -1;
-    pstart[k] = cl[k].pstart;
-    pcount[k] = cl[k].n;
-    parent[k] = -1;
-    level[k] = 0;
-    branch[k] = k;
-  }
-  if (k == 0) {
-    info->nbranch = ncl;
-    info->ctot = ncl - 1;
-    info->first_cell[0] = 0;
-    info->last_cell[0] = ncl - 1;
-  }
-}
-
-__device__ __forceinline__ int key_digit(unsigned long long key, int lev) {
-  return (int)((key >> (3 * (KEY_LEVELS - 1 - lev))) & 7ull);
-}
-
-// the octant digit of level lev+1 of the particle at sorted position i: from
-// the sorted 64-bit keys for the first KEY_LEVELS levels, from the input-order
-// lo words (deep builds) below that
-__device__ __forceinline__ int sorted_digit(const unsigned long long* __restrict__ keys,
-                                            const unsigned* __restrict__ lo,
-                                            const int* __restrict__ idx, int i, int lev) {
-  if (lev < KEY_LEVELS) return key_digit(keys[i], lev);
-  return (int)((lo[idx[i]] >> (3 * (DEEP_LEVELS - 1 - lev))) & 7u);
-}
-
-// children of every branch cell on level lev: boundaries of the octant digit
-// runs inside the cell's (sorted) particle range
-__global__ void k_split(const int* __restrict__ branch, const TreeInfo* __restrict__ info, int lev,
-                        const int* __restrict__ pstart, const int* __restrict__ pcount,
-                        const unsigned long long* __restrict__ keys,
-                        const unsigned* __restrict__ lo_words, const int* __restrict__ idx,
-                        int* __restrict__ nchild, int* __restrict__ cstart) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= info->nbranch) return;
-  const int b = branch[j];
-  const int s = pstart[b], e = s + pcount[b];
-  int st[9];
-  st[0] = s;
-  st[8] = e;
-  for (int d = 1; d < 8; ++d) {
-    int lo = st[d - 1], hi = e;
-    while (lo < hi) {
-      const int mid = lo + ((hi - lo) >> 1);
-      if (sorted_digit(keys, lo_words, idx, mid, lev) < d) lo = mid + 1;
-      else hi = mid;
+// The digit counts of all tiles scanned by one block (few tiles)
+constexpr int RS_SCAN1 = 16384;
+__global__ void __launch_bounds__(1024) k_rs_scan(int* __restrict__ h, int n) {
+  __shared__ int wsum[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int carry = 0;
+  for (int b = 0; b < n; b += 4096) {
+    const int i = b + threadIdx.x * 4;
+    int v[4], t = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      v[j] = i + j < n ? h[i + j] : 0;
+      t += v[j];
     }
-    st[d] = lo;
+    int x = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(FULL, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[w] = x;
+    __syncthreads();
+    if (w == 0) {
+      int y = wsum[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int z = __shfl_up_sync(FULL, y, o);
+        if (lane >= o) y += z;
+      }
+      wsum[lane] = y;
+    }
+    __syncthreads();
+    int e = carry + x - t + (w > 0 ? wsum[w - 1] : 0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (i + j < n) h[i + j] = e;
+      e += v[j];
+    }
+    carry += wsum[31];
+    __syncthreads();
   }
-  int cnt = 0;
-  for (int d = 0; d < 8; ++d) {
-    cstart[j * 9 + d] = st[d];
-    cnt += (st[d + 1] > st[d]) ? 1 : 0;
-  }
-  cstart[j * 9 + 8] = e;
-  nchild[j] = cnt;
 }
 
-// number the children serially in (branch order, octant) order, as
-// BHgrav_build.F90:149-157 does, and link them (:239-253)
-__global__ void k_emit(const int* __restrict__ branch, const TreeInfo* __restrict__ info, int lev,
-                       const int* __restrict__ choff, const int* __restrict__ cstart,
-                       int level_first, int* leaf, int* nextcell, int* ifopen, int* pstart,
-                       int* pcount, int* parent, int* level, int* nkids,
-                       int* __restrict__ bflag) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= info->nbranch) return;
-  const int b = branch[j];
-  const int first = level_first + choff[j];
-  int k = 0, prev = -1;
-  for (int d = 0; d < 8; ++d) {
-    const int s = cstart[j * 9 + d], e = cstart[j * 9 + d + 1];
-    if (e == s) continue;
-    const int c = first + k;
-    ++k;
-    const int cnt = e - s;
-    const int lf = cnt <= LEAFMAX ? cnt : 0;
-    leaf[c] = lf;
-    ifopen[c] = -1;
-    pstart[c] = s;
-    pcount[c] = cnt;
-    parent[c] = b;
-    level[c] = lev + 1;
-    nkids[c] = 0;
-    bflag[c - level_first] = lf == 0 ? 1 : 0;
-    if (prev >= 0) nextcell[prev] = c;
-    prev = c;
+// Sort of at most SS_MAX (key, index) pairs by one block: bitonic on (key, index),
+// so equal keys keep their input order.  777 particles: 12 us, where the 8 digit
+// passes of the radix sort take 230.
+constexpr int SS_MAX = 4096;
+constexpr int SS_T = 1024;
+__global__ void __launch_bounds__(SS_T) k_small_sort(unsigned long long* __restrict__ keys,
+                                                     int* __restrict__ idx, int n) {
+  extern __shared__ __align__(16) unsigned char ss_buf[];
+  int N = 2;
+  while (N < n) N <<= 1;
+  unsigned long long* sk = reinterpret_cast<unsigned long long*>(ss_buf);
+  int* sv = reinterpret_cast<int*>(sk + N);
+  for (int i = threadIdx.x; i < N; i += SS_T) {
+    sk[i] = i < n ? keys[i] : ~0ull;
+    sv[i] = i < n ? idx[i] : 0x7fffffff;
   }
-  nextcell[prev] = nextcell[b];
-  ifopen[b] = first;
-  nkids[b] = k;
-}
-
-__global__ void k_next_branch(const int* __restrict__ bflag, const int* __restrict__ bscan, int nnew,
-                              int level_first, int* __restrict__ branch_next) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nnew) return;
-  if (bflag[i]) branch_next[bscan[i]] = level_first + i;
-}
-
-__global__ void k_level_done(TreeInfo* info, int lev, int level_first, int nnew,
-                             const int* __restrict__ nb_next) {
-  info->ctot = level_first + nnew - 1;
-  info->first_cell[lev + 1] = level_first;
-  info->last_cell[lev + 1] = level_first + nnew - 1;
-  info->ltot = lev + 1;
-  info->nbranch = *nb_next;
-  info->nchild = nnew;
-}
-
-// leaf particles back to input-index order (the linked lists of the
-// reference keep the order particles had in the parent cell, and the root
-// list is 1..ptot), then the permutation new -> old
-__global__ void k_leaf_order(const int* __restrict__ leaf, const int* __restrict__ pstart, int ctot,
-                             int* __restrict__ idx) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c > ctot) return;
-  const int n = leaf[c];
-  if (n <= 1) return;
-  const int s = pstart[c];
-  int v[LEAFMAX];
-  for (int i = 0; i < n; ++i) v[i] = idx[s + i];
-  for (int i = 1; i < n; ++i) {
-    const int x = v[i];
-    int j = i - 1;
-    while (j >= 0 && v[j] > x) { v[j + 1] = v[j]; --j; }
-    v[j + 1] = x;
+  __syncthreads();
+  for (int size = 2; size <= N; size <<= 1)
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int i = threadIdx.x; i < (N >> 1); i += SS_T) {
+        const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
+        const unsigned long long a = sk[lo], b = sk[hi];
+        const int va = sv[lo], vb = sv[hi];
+        if ((a > b || (a == b && va > vb)) == ((lo & size) == 0)) {
+          sk[lo] = b; sk[hi] = a;
+          sv[lo] = vb; sv[hi] = va;
+        }
+      }
+      __syncthreads();
+    }
+  for (int i = threadIdx.x; i < n; i += SS_T) {
+    keys[i] = sk[i];
+    idx[i] = sv[i];
   }
-  for (int i = 0; i < n; ++i) idx[s + i] = v[i];
+}
+
+// ---------------------------------------------------------------------------
+// The cells from the sorted keys, all levels at once.  With share(i, j) the
+// number of leading octants particles i and j have in common (-1 in different
+// clouds; sorted order), the cells of level L are the runs of a common L-octant
+// prefix inside a split cell (more than LEAFMAX particles, or a root), so:
+//  * particle i's leaf is on the first level whose run has at most LEAFMAX
+//    particles: leaf(i) = 1 + the largest share(j, j + 8) over j = i-8..i (at least
+//    1, since a root is always split, BHgrav_build.F90:74);
+//  * i starts cells on the levels share(i-1, i) + 1 .. leaf(i);
+//  * the children of every level are numbered serially in (parent, octant) order
+//    (:149-157), which is the sorted order, so a cell's number is its level's first
+//    plus the starts of that level before it.
+// k_cells_mark writes each particle's start levels as a bit mask and counts them
+// per block, k_cells_scan turns the counts into offsets, and k_cells_emit
+// writes every cell: 3 launches and one host read (the level sizes) where a level-by-
+// level split took 10 and 2 for each level (60-70 us a level).
+constexpr int CE_T = 256;
+
+// Sorted keys: levels 1..21 in keys, 22..30 in lo (input order, with deep); levels
+// beyond `ordered` are not sorted and count as shared.
+struct SortedKeys {
+  const unsigned long long* keys;
+  const unsigned* lo;
+  const int* idx;
+  int deep;
+  int ordered;
+};
+
+__device__ __forceinline__ int share_levels(unsigned long long a, unsigned long long b,
+                                            unsigned la, unsigned lb, const SortedKeys& k) {
+  const unsigned long long x = a ^ b;
+  int c = x == 0ull ? KEY_LEVELS : (__clzll(x) - 1) / 3;
+  if (x == 0ull && k.deep) {
+    const unsigned y = la ^ lb;
+    c += y == 0u ? LO_LEVELS : (__clz(y) - 5) / 3;
+  }
+  return min(c, k.ordered);
+}
+
+__global__ void __launch_bounds__(CE_T) k_cells_mark(int n, SortedKeys K,
+                                                     const CloudInfo* __restrict__ cl, int ncl,
+                                                     unsigned* __restrict__ mask,
+                                                     int* __restrict__ blk_count, int nblk) {
+  constexpr int H = LEAFMAX;
+  __shared__ unsigned long long sk[CE_T + 2 * H];
+  __shared__ unsigned sl[CE_T + 2 * H];
+  __shared__ int sc[CE_T + 2 * H];
+  __shared__ int s8[CE_T + H];           // share(j, j + 8), j from base - 8
+  __shared__ int cnt[32];
+  const int base = blockIdx.x * CE_T;
+  if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
+  for (int t = threadIdx.x; t < CE_T + 2 * H; t += CE_T) {
+    const int i = base - H + t;
+    const bool in = i >= 0 && i < n;
+    sk[t] = in ? K.keys[i] : 0ull;
+    sl[t] = in && K.deep ? K.lo[K.idx[i]] : 0u;
+    sc[t] = !in ? -1 : cl ? cloud_of(cl, ncl, i) : 0;
+  }
+  __syncthreads();
+  auto share = [&](int a, int b) {
+    if (sc[a] < 0 || sc[a] != sc[b]) return -1;
+    return share_levels(sk[a], sk[b], sl[a], sl[b], K);
+  };
+  for (int t = threadIdx.x; t < CE_T + H; t += CE_T) s8[t] = share(t, t + H);
+  __syncthreads();
+  const int i = base + threadIdx.x;
+  unsigned m = 0u;
+  if (i < n) {
+    int c8 = 0;
+#pragma unroll
+    for (int j = 0; j <= H; ++j) c8 = max(c8, s8[threadIdx.x + j]);
+    const int l0 = share(threadIdx.x + H - 1, threadIdx.x + H);
+    const int leaf = c8 + 1;                           // (c8 >= 0: level 1 at least)
+    if (l0 < leaf) m = (leaf >= 31 ? FULL : (2u << leaf) - 1u) & ~((1u << (l0 + 1)) - 1u);
+    mask[i] = m;
+  }
+  for (int l = 0; l < 32; ++l) {
+    const unsigned b = __ballot_sync(FULL, (m >> l) & 1u);
+    if ((threadIdx.x & 31) == 0 && b) atomicAdd(&cnt[l], __popc(b));
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) blk_count[threadIdx.x * nblk + blockIdx.x] = cnt[threadIdx.x];
+}
+
+// block l: the exclusive scan of level l's block counts, its total to info->ncell[l]
+__global__ void __launch_bounds__(1024) k_cells_scan(int* __restrict__ blk_count, int nblk,
+                                                     TreeInfo* info) {
+  __shared__ int wsum[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int* h = blk_count + (size_t)blockIdx.x * nblk;
+  int carry = 0;
+  for (int b = 0; b < nblk; b += 1024) {
+    const int i = b + threadIdx.x;
+    const int v = i < nblk ? h[i] : 0;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(FULL, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[w] = x;
+    __syncthreads();
+    if (w == 0) {
+      int y = wsum[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int z = __shfl_up_sync(FULL, y, o);
+        if (lane >= o) y += z;
+      }
+      wsum[lane] = y;
+    }
+    __syncthreads();
+    if (i < nblk) h[i] = carry + x - v + (w > 0 ? wsum[w - 1] : 0);
+    carry += wsum[31];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) info->ncell[blockIdx.x] = carry;
+}
+
+struct LevelFirst {
+  int first[33];
+};
+
+__global__ void __launch_bounds__(CE_T) k_cells_emit(
+    int n, SortedKeys K, const CloudInfo* __restrict__ cl, int ncl,
+    const unsigned* __restrict__ mask, const int* __restrict__ blk_count, int nblk, int ltot,
+    LevelFirst F, int cmax, int* __restrict__ idx, int4* __restrict__ link,
+    int* __restrict__ pcount, int* __restrict__ parent, int* __restrict__ level,
+    int* __restrict__ nkids) {
+  __shared__ unsigned wb[CE_T / 32][32];   // starts of a level in a warp
+  __shared__ int wpre[CE_T / 32][32];      // starts of the level before the warp
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = blockIdx.x * CE_T + threadIdx.x;
+  const unsigned m = i < n ? mask[i] : 0u;
+  for (int l = 0; l <= ltot; ++l) {
+    const unsigned b = __ballot_sync(FULL, (m >> l) & 1u);
+    if (lane == 0) wb[w][l] = b;
+  }
+  __syncthreads();
+  if (threadIdx.x <= ltot) {
+    int run = blk_count[threadIdx.x * nblk + blockIdx.x];
+    for (int ww = 0; ww < CE_T / 32; ++ww) {
+      wpre[ww][threadIdx.x] = run;
+      run += __popc(wb[ww][threadIdx.x]);
+    }
+  }
+  __syncthreads();
+  if (m == 0u) return;
+  // the level-l cell that starts at i, or would next
+  auto number = [&](int l) {
+    return F.first[l] + wpre[w][l] + __popc(wb[w][l] & ((1u << lane) - 1u));
+  };
+  int hi = n;                              // the end of the cell above
+  if (cl) {
+    const CloudInfo& C = cl[cloud_of(cl, ncl, i)];
+    hi = C.pstart + C.n;
+  }
+  const int cloud_end = hi;
+  const int l0 = __ffs(m) - 1, leaf = 31 - __clz(m);
+  const unsigned long long key = K.keys[i];
+  const unsigned lo = K.deep ? K.lo[K.idx[i]] : 0u;
+  for (int l = l0; l <= leaf; ++l) {
+    int end;
+    if (l == 0) {
+      end = cloud_end;
+    } else if (l == leaf) {                // the next start of this level or above it
+      end = i + 1;
+      while (end < hi && (mask[end] & ((2u << l) - 1u)) == 0u) ++end;
+    } else {                               // more than LEAFMAX: the end of the prefix
+      int a = i + LEAFMAX + 1, b = hi;
+      while (a < b) {
+        const int mid = a + ((b - a) >> 1);
+        if (share_levels(key, K.keys[mid], lo, K.deep ? K.lo[K.idx[mid]] : 0u, K) >= l) a = mid + 1;
+        else b = mid;
+      }
+      end = a;
+    }
+    const int c = number(l);
+    // next cell: the one that starts at `end` below the deepest ancestor (or
+    // self) level both share, which follows the cell of that level holding i
+    int next = cmax + 1;                                             // BHgrav_build.F90:75
+    if (end < cloud_end) {
+      const int ln = __ffs(mask[end]) - 1;                           // <= l
+      next = number(ln) + (ln >= l0 ? 1 : 0);
+    }
+    // parent: started here too, or the last one of its level before i
+    const int par = l == 0 ? -1 : l > l0 ? number(l - 1) : number(l - 1) - 1;
+    const bool isleaf = l == leaf;
+    link[c] = make_int4(isleaf ? end - i : 0, next, isleaf ? -1 : number(l + 1), i);
+    pcount[c] = end - i;
+    parent[c] = par;
+    level[c] = l;
+    if (par >= 0) atomicAdd(nkids + par, 1);
+    hi = end;
+  }
+  // the leaf's particles back to input-index order (the linked lists of the
+  // reference keep the order particles had in the parent cell, and the root
+  // list is 1..ptot)
+  const int cnt = hi - i;
+  if (cnt > 1) {
+    int v[LEAFMAX];
+    for (int k = 0; k < cnt; ++k) v[k] = idx[i + k];
+    for (int k = 1; k < cnt; ++k) {
+      const int x = v[k];
+      int j = k - 1;
+      while (j >= 0 && v[j] > x) { v[j + 1] = v[j]; --j; }
+      v[j + 1] = x;
+    }
+    for (int k = 0; k < cnt; ++k) idx[i + k] = v[k];
+  }
 }
 
 __global__ void k_reorder(const int* __restrict__ perm, int n, const double4* __restrict__ pm,
@@ -589,14 +743,6 @@ __global__ void k_reorder_rk(const int* __restrict__ perm, int n, const double4*
   c2[i] = c[p];
 }
 
-__global__ void k_pack_link(int ctot, const int* __restrict__ leaf, const int* __restrict__ nextcell,
-                            const int* __restrict__ ifopen, const int* __restrict__ pstart,
-                            int4* __restrict__ link) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c > ctot) return;
-  link[c] = make_int4(leaf[c], nextcell[c], leaf[c] > 0 ? -1 : ifopen[c], pstart[c]);
-}
-
 __global__ void k_unpack_parray(const double* __restrict__ st, int n, double4* __restrict__ pm,
                                 double2* __restrict__ hz, DevError* err) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -628,7 +774,7 @@ __global__ void k_pack_parray(double* __restrict__ st, int n, const double4* __r
 // rounding of the walk's prefilter test (coordinates rounded to within delta,
 // the difference, the squares and the sum); tests inside the bracket are
 // redone in FP64 by the walk.
-__global__ void k_stock_level(int cfirst, int clast, const int4* __restrict__ link,
+__device__ __forceinline__ void stock_cell(int c, const int4* __restrict__ link,
                               const double4* __restrict__ pm, const double2* __restrict__ hz,
                               double thetamaxsqd, double daux, double4* __restrict__ gA,
                               double4* __restrict__ gB, double2* __restrict__ gC,
@@ -638,8 +784,6 @@ __global__ void k_stock_level(int cfirst, int clast, const int4* __restrict__ li
                               const int* __restrict__ nkids, float4* __restrict__ wA,
                               float4* __restrict__ hA32, float4* __restrict__ hN,
                               const CloudInfo* __restrict__ cl, int ncl) {
-  const int c = cfirst + blockIdx.x * blockDim.x + threadIdx.x;
-  if (c > clast) return;
   const int4 lk = link[c];
   if (cl) {                                  // a forest: the cell's own cloud's root box
     const CloudInfo& C = cl[cloud_of(cl, ncl, lk.w)];
@@ -686,9 +830,8 @@ __global__ void k_stock_level(int cfirst, int clast, const int4* __restrict__ li
       qc[4] = qc[4] + mp * ((3.0 * dr[2]) * dr[1]);
     }
   } else {                                                           // :188-312
-    const int cend = lk.y;
-    int cc = lk.z;
-    while (true) {
+    const int cfirst = lk.z, cend = lk.z + nkids[c];   // children are consecutive cells
+    for (int cc = cfirst; cc < cend; ++cc) {
       const double4 a = gA[cc];
       mc = mc + a.w;
       rc[0] = rc[0] + a.w * a.x;
@@ -699,12 +842,9 @@ __global__ void k_stock_level(int cfirst, int clast, const int4* __restrict__ li
       bbmax[0] = fmax(b1.x, bbmax[0]); bbmin[0] = fmin(b0.x, bbmin[0]);
       bbmax[1] = fmax(b1.y, bbmax[1]); bbmin[1] = fmin(b0.y, bbmin[1]);
       bbmax[2] = fmax(b1.z, bbmax[2]); bbmin[2] = fmin(b0.z, bbmin[2]);
-      cc = link[cc].y;
-      if (cc == cend) break;
     }
     if (mc > 0.0) for (int k = 0; k < 3; ++k) rc[k] = rc[k] / mc;
-    cc = lk.z;
-    while (true) {
+    for (int cc = cfirst; cc < cend; ++cc) {
       const double4 a = gA[cc];
       const double4 q = gB[cc];
       const double2 q5 = gC[cc];
@@ -718,8 +858,6 @@ __global__ void k_stock_level(int cfirst, int clast, const int4* __restrict__ li
       qc[2] = qc[2] + mcc * ((3.0 * dr[1]) * dr[1] - drsqd);
       qc[3] = qc[3] + mcc * ((3.0 * dr[2]) * dr[0]);
       qc[4] = qc[4] + mcc * ((3.0 * dr[2]) * dr[1]);
-      cc = link[cc].y;
-      if (cc == cend) break;
     }
   }
   // MAC quantities, :317-348
@@ -765,30 +903,81 @@ __global__ void k_stock_level(int cfirst, int clast, const int4* __restrict__ li
                               __int_as_float(lk.x > 0 ? lk.x : -nkids[c]), 0.0f);
 }
 
-// BHhydro_update_hmax.F90:29-88
-__global__ void k_hmax_level(int cfirst, int clast, const int4* __restrict__ link,
-                             const double2* __restrict__ hz, double* __restrict__ hrm,
-                             float* __restrict__ hrm32, float4* __restrict__ hN) {
+// The cells [cfirst, clast] of one level; or (levels > 1) the levels
+// `levels`-1 .. 0 by one block, one after another: the upper levels are few cells
+// each, and a launch of its own for each of them is all latency.
+struct StockArgs {
+  const int4* link;
+  const double4* pm;
+  const double2* hz;
+  double thetamaxsqd, daux;
+  double4* gA;
+  double4* gB;
+  double2* gC;
+  double4* hA;
+  double* hmaxa;
+  double4* bbmina;
+  double4* bbmaxa;
+  double rootx, rooty, rootz, delta;
+  const int* nkids;
+  float4* wA;
+  float4* hA32;
+  float4* hN;
+  const CloudInfo* cl;
+  int ncl;
+};
+__device__ __forceinline__ void stock_one(int c, const StockArgs& a) {
+  stock_cell(c, a.link, a.pm, a.hz, a.thetamaxsqd, a.daux, a.gA, a.gB, a.gC, a.hA, a.hmaxa,
+             a.bbmina, a.bbmaxa, a.rootx, a.rooty, a.rootz, a.delta, a.nkids, a.wA, a.hA32, a.hN,
+             a.cl, a.ncl);
+}
+__global__ void k_stock_level(int cfirst, int clast, StockArgs a) {
   const int c = cfirst + blockIdx.x * blockDim.x + threadIdx.x;
-  if (c > clast) return;
+  if (c <= clast) stock_one(c, a);
+}
+constexpr int TOP_T = 512;
+constexpr int TOP_CELLS = 1024;      // cells of a level that the one-block kernels take
+__global__ void __launch_bounds__(TOP_T) k_stock_top(int levels, LevelFirst F, StockArgs a) {
+  for (int l = levels - 1; l >= 0; --l) {
+    for (int c = F.first[l] + threadIdx.x; c < F.first[l + 1]; c += TOP_T) stock_one(c, a);
+    __syncthreads();
+  }
+}
+
+// BHhydro_update_hmax.F90:29-88
+__device__ __forceinline__ void hmax_cell(int c, const int4* __restrict__ link,
+                                          const int* __restrict__ nkids,
+                                          const double2* __restrict__ hz, double* hrm,
+                                          float* __restrict__ hrm32, float4* __restrict__ hN) {
   const int4 lk = link[c];
   double hr = 0.0;
-  if (lk.x == 1) {
-    hr = KERNRANGE * hz[lk.w].x;
-  } else if (lk.x > 0) {
+  if (lk.x > 0) {
     for (int i = 0; i < lk.x; ++i) hr = fmax(hr, KERNRANGE * hz[lk.w + i].x);
   } else {
-    int cc = lk.z;
-    const int cend = lk.y;
-    while (true) {
-      hr = fmax(hr, hrm[cc]);
-      cc = link[cc].y;
-      if (cc == cend) break;
-    }
+    const int nk = nkids[c];
+    for (int k = 0; k < nk; ++k) hr = fmax(hr, hrm[lk.z + k]);
   }
   hrm[c] = hr;
   hrm32[c] = __double2float_ru(hr);
   reinterpret_cast<float*>(hN)[8 * (size_t)c + 4] = hrm32[c];
+}
+__global__ void k_hmax_level(int cfirst, int clast, const int4* __restrict__ link,
+                             const int* __restrict__ nkids, const double2* __restrict__ hz,
+                             double* hrm, float* __restrict__ hrm32, float4* __restrict__ hN) {
+  const int c = cfirst + blockIdx.x * blockDim.x + threadIdx.x;
+  if (c <= clast) hmax_cell(c, link, nkids, hz, hrm, hrm32, hN);
+}
+__global__ void __launch_bounds__(TOP_T) k_hmax_top(int levels, LevelFirst F,
+                                                    const int4* __restrict__ link,
+                                                    const int* __restrict__ nkids,
+                                                    const double2* __restrict__ hz, double* hrm,
+                                                    float* __restrict__ hrm32,
+                                                    float4* __restrict__ hN) {
+  for (int l = levels - 1; l >= 0; --l) {
+    for (int c = F.first[l] + threadIdx.x; c < F.first[l + 1]; c += TOP_T)
+      hmax_cell(c, link, nkids, hz, hrm, hrm32, hN);
+    __syncthreads();
+  }
 }
 
 // BHhydro_hguess.F90:106-155 (GRAD_H_SPH number criterion): the h of a
@@ -895,79 +1084,98 @@ void launch_pack_parray(Ctx& c, double* stage, int n, cudaStream_t s) {
   k_pack_parray<<<nb(n, 256), 256, 0, s ? s : c.st>>>(stage, n, c.pm, c.hz); ++c.nlaunch;
 }
 
-// stable LSD sort of (keys, idx) on the key bits [0, bits), 8 at a time; an
-// even number of passes leaves the sorted data in keys/idx
-static void radix_sort(Ctx& c, int n, int bits) {
+template <int RS_I>
+static void radix_passes(Ctx& c, int n, int lo, int bits) {
   static bool smem_set[16] = {};   // the scatter's shared memory is above the 48 KB default
   bool& ss = smem_set[c.dev >= 0 && c.dev < 16 ? c.dev : 0];
   if (!ss) {
-    cudaFuncSetAttribute(k_rs_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SMEM);
+    cudaFuncSetAttribute(k_rs_scatter<RS_I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)rs_smem(RS_I));
     ss = true;
   }
-  const int nblk = nb(n, RS_TILE);
+  const int nblk = nb(n, RS_T * RS_I);
   unsigned long long* ka = c.keys;
   unsigned long long* kb = c.keys_alt;
   int* va = c.idx;
   int* vb = c.idx_alt;
-  for (int shift = 0; shift < bits; shift += 8) {
-    k_rs_hist<<<nblk, RS_T, 0, c.st>>>(ka, n, shift, c.rs_hist, nblk); ++c.nlaunch;
-    scan_exclusive(c, c.rs_hist, c.rs_hist, 256 * nblk);
-    k_rs_scatter<<<nblk, RS_T, RS_SMEM, c.st>>>(ka, va, kb, vb, n, shift, c.rs_hist, nblk);
+  for (int shift = lo; shift < bits; shift += 8) {
+    k_rs_hist<RS_I><<<nblk, RS_T, 0, c.st>>>(ka, n, shift, c.rs_hist, nblk); ++c.nlaunch;
+    if (256 * nblk <= RS_SCAN1) {
+      k_rs_scan<<<1, 1024, 0, c.st>>>(c.rs_hist, 256 * nblk); ++c.nlaunch;
+    } else {
+      scan_exclusive(c, c.rs_hist, c.rs_hist, 256 * nblk);
+    }
+    k_rs_scatter<RS_I><<<nblk, RS_T, rs_smem(RS_I), c.st>>>(ka, va, kb, vb, n, shift, c.rs_hist,
+                                                            nblk);
     ++c.nlaunch;
     std::swap(ka, kb);
     std::swap(va, vb);
   }
 }
 
-constexpr int NEED_DEEP_KEYS = -1;
+size_t radix_hist_ints(size_t pmax) {
+  const size_t small = std::min<size_t>(pmax, RS_SMALL);
+  return 256 * std::max((pmax + RS_T * 16 - 1) / (RS_T * 16), (small + RS_T * 4 - 1) / (RS_T * 4));
+}
 
-// cells level by level from the sorted keys; with 21-level keys, a tree that
-// needs level 22 returns NEED_DEEP_KEYS
-static int build_cells(Ctx& c, bool deep, int& ctot_out) {
+// stable sort of (keys, idx) on the key bits [lo, bits), 8 at a time; an even
+// number of passes leaves the sorted data in keys/idx.  Few items: one block
+// sorts on all bits (idx holds the input order of equal keys in increasing order).
+static void radix_sort(Ctx& c, int n, int lo, int bits) {
+  if (n < RS_SMALL) radix_passes<4>(c, n, lo, bits);
+  else radix_passes<16>(c, n, lo, bits);
+}
+
+constexpr int NEED_MORE_LEVELS = -1;
+
+// the cells of the sorted keys (`ordered` levels of them); NEED_MORE_LEVELS when
+// a cell on level `ordered` has to be split
+static int build_cells(Ctx& c, bool deep, int ordered) {
   const int n = c.ptot;
   const int ncl = c.ncloud;
-  if (ncl > 1)
-    k_roots<<<nb(ncl, 128), 128, 0, c.st>>>(ncl, c.d_clouds, c.cmax, c.leaf, c.nextcell, c.ifopen,
-                                            c.pstart, c.pcount, c.parent, c.level, c.branch,
-                                            c.d_info);
-  else
-    k_root<<<1, 1, 0, c.st>>>(n, c.cmax, c.leaf, c.nextcell, c.ifopen, c.pstart, c.pcount,
-                              c.parent, c.level, c.branch, c.d_info);
-  ++c.nlaunch;
-  int nbranch = ncl, ctot = ncl - 1, lev = 0;
-  int* br = c.branch;
-  int* br_next = c.branch_next;
+  const CloudInfo* cl = ncl > 1 ? c.d_clouds : nullptr;
+  const SortedKeys K{c.keys, c.keys_lo, c.idx, deep ? 1 : 0, ordered};
+  unsigned* mask = reinterpret_cast<unsigned*>(c.idx_alt);      // free after the sort
+  const int nblk = nb(n, CE_T);
+  k_cells_mark<<<nblk, CE_T, 0, c.st>>>(n, K, cl, ncl, mask, c.blk_count, nblk);
+  k_cells_scan<<<32, 1024, 0, c.st>>>(c.blk_count, nblk, c.d_info);
+  c.nlaunch += 2;
+  TreeInfo info;
+  static_assert(sizeof(TreeInfo) % 4 == 0 && sizeof(TreeInfo) <= 1024, "TreeInfo through read_dev");
+  if (read_dev(c, c.d_info, &info, sizeof(TreeInfo))) return SEREN_GPU_ERR_CUDA;
+  // the levels in turn, with the reference's limits (level lev has cells to
+  // split when level lev + 1 has cells)
+  LevelFirst F{};
+  int ctot = ncl - 1, lev = 0;
+  F.first[0] = 0;
+  F.first[1] = ncl;
+  info.first_cell[0] = 0;
+  info.last_cell[0] = ncl - 1;
   while (true) {
     if (lev >= c.prm.lmax) {                // BHgrav_build.F90:289
       c.err = "Reached maximum level (tree deeper than lmax)";
       return SEREN_GPU_ERR_LMAX;
     }
-    if (!deep && lev >= KEY_LEVELS) return NEED_DEEP_KEYS;
-    k_split<<<nb(nbranch, 128), 128, 0, c.st>>>(br, c.d_info, lev, c.pstart, c.pcount, c.keys,
-                                                c.keys_lo, c.idx, c.nchild, c.cstart); ++c.nlaunch;
-    scan_exclusive(c, c.nchild, c.choff, nbranch);
-    int nnew = 0;
-    if (read_dev(c, c.scan.total, &nnew, sizeof(int))) return SEREN_GPU_ERR_CUDA;
-    const int level_first = ctot + 1;
+    if (lev >= ordered && ordered < DEEP_LEVELS) return NEED_MORE_LEVELS;
+    const int nnew = info.ncell[lev + 1];
     if ((long)ctot + nnew > (long)c.cmax) {
       c.err = "cell count exceeds cmax = 2*pmax";
       return SEREN_GPU_ERR_CAPACITY;
     }
-    k_emit<<<nb(nbranch, 128), 128, 0, c.st>>>(br, c.d_info, lev, c.choff, c.cstart, level_first,
-                                               c.leaf, c.nextcell, c.ifopen, c.pstart, c.pcount,
-                                               c.parent, c.level, c.nkids, c.bflag); ++c.nlaunch;
-    scan_exclusive(c, c.bflag, c.bscan, nnew);
-    k_next_branch<<<nb(nnew, 256), 256, 0, c.st>>>(c.bflag, c.bscan, nnew, level_first, br_next); ++c.nlaunch;
-    k_level_done<<<1, 1, 0, c.st>>>(c.d_info, lev, level_first, nnew, c.scan.total); ++c.nlaunch;
-    int nbn = 0;
-    if (read_dev(c, c.scan.total, &nbn, sizeof(int))) return SEREN_GPU_ERR_CUDA;
+    info.first_cell[lev + 1] = ctot + 1;
+    info.last_cell[lev + 1] = ctot + nnew;
     ctot += nnew;
     ++lev;
-    std::swap(br, br_next);
-    nbranch = nbn;
-    if (nbranch == 0) break;
+    F.first[lev + 1] = ctot + 1;
+    if (lev >= 31 || info.ncell[lev + 1] == 0) break;
   }
-  ctot_out = ctot;
+  info.ctot = ctot;
+  info.ltot = lev;
+  cudaMemsetAsync(c.nkids, 0, sizeof(int) * ((size_t)ctot + 1), c.st);
+  k_cells_emit<<<nblk, CE_T, 0, c.st>>>(n, K, cl, ncl, mask, c.blk_count, nblk, lev, F, c.cmax,
+                                        c.idx, c.link, c.pcount, c.parent, c.level, c.nkids);
+  ++c.nlaunch;
+  c.info = info;
   return SEREN_GPU_OK;
 }
 
@@ -976,7 +1184,7 @@ static int build_cells(Ctx& c, bool deep, int& ctot_out) {
 // are gathered into that order for the cell split
 static void sort_by_cloud(Ctx& c, int n) {
   k_cloud_keys<<<nb(n, 256), 256, 0, c.st>>>(c.idx, n, c.d_clouds, c.ncloud, c.keys); ++c.nlaunch;
-  radix_sort(c, n, c.ncloud <= 65536 ? 16 : 32);      // an even number of passes
+  radix_sort(c, n, 0, c.ncloud <= 65536 ? 16 : 32);   // an even number of passes
   k_gather_hi<<<nb(n, 256), 256, 0, c.st>>>(c.keys_hi, c.idx, n, c.keys); ++c.nlaunch;
 }
 
@@ -985,31 +1193,60 @@ int build_tree(Ctx& c) {
   const bool forest = c.ncloud > 1;
   const CloudInfo* cl = forest ? c.d_clouds : nullptr;
   if (forest) {
-    k_bbox_clouds<<<c.ncloud, BB_T, 0, c.st>>>(c.pm, c.d_clouds, c.d_info); ++c.nlaunch;
+    // (the keys' second buffer holds the slices: 6 doubles each, at most n of them)
+    const int ns = std::max(1, std::min({64, 4096 / c.ncloud, n / (6 * c.ncloud)}));
+    double* part = c.ncloud * 6 <= n ? reinterpret_cast<double*>(c.keys_alt) : c.stage;
+    k_bbox_cloud_part<<<dim3(c.ncloud, ns), BB_T, 0, c.st>>>(c.pm, c.d_clouds, part);
+    k_bbox_clouds<<<nb(c.ncloud, 128), 128, 0, c.st>>>(c.ncloud, ns, part, c.d_clouds, c.d_info);
+    c.nlaunch += 2;
   } else {
     const int bblk = std::min(nb(n, BB_T), 1184);
     k_bbox_partial<<<bblk, BB_T, 0, c.st>>>(c.pm, n, c.bbox_part); ++c.nlaunch;
     k_bbox_final<<<1, BB_T, 0, c.st>>>(c.bbox_part, bblk, c.d_info); ++c.nlaunch;
   }
-  k_keys<<<nb(n, 256), 256, 0, c.st>>>(c.pm, n, c.d_info, cl, c.ncloud, c.keys,
-                                        forest ? c.keys_hi : nullptr, c.idx); ++c.nlaunch;
-  radix_sort(c, n, 64);
-  if (forest) sort_by_cloud(c, n);
-  int ctot = 0;
-  int rc = build_cells(c, false, ctot);
-  if (rc == NEED_DEEP_KEYS) {
+  auto keys = [&]() {
+    k_keys<<<nb(n, 256), 256, 0, c.st>>>(c.pm, n, c.d_info, cl, c.ncloud, c.keys,
+                                          forest ? c.keys_hi : nullptr, c.idx); ++c.nlaunch;
+  };
+  // The key's upper 32 bits order 10 levels in 4 passes, enough for most trees (a
+  // uniform cloud of 2^28 particles has 10); a tree that needs more is sorted
+  // again on all of them, at once where the last one did (c.deep_sort).
+  keys();
+  int rc = NEED_MORE_LEVELS;
+  if (n <= SS_MAX && !forest) {
+    int N = 2;
+    while (N < n) N <<= 1;
+    k_small_sort<<<1, SS_T, (size_t)N * 12, c.st>>>(c.keys, c.idx, n); ++c.nlaunch;
+    rc = build_cells(c, false, KEY_LEVELS);
+  } else {
+    if (!c.deep_sort) {
+      radix_sort(c, n, 31, 63);
+      if (forest) sort_by_cloud(c, n);
+      rc = build_cells(c, false, 10);
+      if (rc == NEED_MORE_LEVELS) {
+        c.deep_sort = true;
+        keys();
+      }
+    }
+    if (rc == NEED_MORE_LEVELS) {
+      radix_sort(c, n, 0, 64);
+      if (forest) sort_by_cloud(c, n);
+      rc = build_cells(c, false, KEY_LEVELS);
+      if (rc == SEREN_GPU_OK) c.deep_sort = c.info.ltot > 10;
+    }
+  }
+  if (rc == NEED_MORE_LEVELS) {
     // sort on (levels 1..21, levels 22..30): stable passes on the low word,
     // then on the high word in that order
     k_keys_deep<<<nb(n, 256), 256, 0, c.st>>>(c.pm, n, c.d_info, cl, c.ncloud, c.keys, c.keys_hi,
                                                c.keys_lo, c.idx); ++c.nlaunch;
-    radix_sort(c, n, 32);
+    radix_sort(c, n, 0, 32);
     k_gather_hi<<<nb(n, 256), 256, 0, c.st>>>(c.keys_hi, c.idx, n, c.keys); ++c.nlaunch;
-    radix_sort(c, n, 64);
+    radix_sort(c, n, 0, 64);
     if (forest) sort_by_cloud(c, n);
-    rc = build_cells(c, true, ctot);
+    rc = build_cells(c, true, DEEP_LEVELS);
   }
   if (rc) return rc;
-  k_leaf_order<<<nb(ctot + 1, 256), 256, 0, c.st>>>(c.leaf, c.pstart, ctot, c.idx); ++c.nlaunch;
   if (c.reorder_wait) {                     // velocities and c_s^2 still being copied in
     k_reorder_pos<<<nb(n, 256), 256, 0, c.st>>>(c.idx, n, c.pm, c.hz, c.orig, c.pm_alt, c.hz_alt,
                                                  c.orig_alt); ++c.nlaunch;
@@ -1040,10 +1277,6 @@ int build_tree(Ctx& c) {
     std::swap(c.v_half, c.v_half_alt);
   }
   if (c.blk.on) reorder_block(c);           // block-timestep state, a and gpot too
-  k_pack_link<<<nb(ctot + 1, 256), 256, 0, c.st>>>(ctot, c.leaf, c.nextcell, c.ifopen, c.pstart,
-                                                   c.link); ++c.nlaunch;
-  static_assert(sizeof(TreeInfo) % 4 == 0 && sizeof(TreeInfo) <= 1024, "TreeInfo through read_dev");
-  if (read_dev(c, c.d_info, &c.info, sizeof(TreeInfo))) return SEREN_GPU_ERR_CUDA;
   c.have_tree = true;
   return SEREN_GPU_OK;
 }
@@ -1091,32 +1324,46 @@ int restock(Ctx& c, bool& rebuilt) {
   return SEREN_GPU_OK;
 }
 
+// the levels 0 .. top-1 with at most TOP_CELLS cells each (level 0 always)
+static int top_levels(const Ctx& c) {
+  int top = 1;
+  while (top <= c.info.ltot && c.info.last_cell[top] - c.info.first_cell[top] < TOP_CELLS) ++top;
+  return top;
+}
+
+static LevelFirst level_first(const Ctx& c, int top) {
+  LevelFirst F{};
+  for (int l = 0; l < top; ++l) F.first[l] = c.info.first_cell[l];
+  F.first[top] = c.info.last_cell[top - 1] + 1;
+  return F;
+}
+
 void launch_stock(Ctx& c) {
   const double daux = 10.0 * pow(1.7976931348623157e308, -0.2);
   // bound on the rounding of a coordinate relative to the root centre when
   // cast to FP32: every position lies within cellsize (the root half width)
   // of the centre on each axis, so half an ulp is below 2^-23 * cellsize
   const double delta = ldexp(1.0, -22) * (c.info.cellsize > 0.0 ? c.info.cellsize : 1.0);
-  for (int l = c.info.ltot; l >= 0; --l) {
+  const StockArgs a{c.link, c.pm, c.hz, c.prm.thetamaxsqd, daux, c.gA, c.gB, c.gC, c.hA, c.hmax,
+                    c.bbmin, c.bbmax, c.info.root[0], c.info.root[1], c.info.root[2], delta,
+                    c.nkids, c.wA, c.hA32, c.hN, c.ncloud > 1 ? c.d_clouds : nullptr, c.ncloud};
+  const int top = top_levels(c);
+  for (int l = c.info.ltot; l >= top; --l) {
     const int f = c.info.first_cell[l], la = c.info.last_cell[l];
-    const int cnt = la - f + 1;
-    if (cnt <= 0) continue;
-    k_stock_level<<<nb(cnt, 128), 128, 0, c.st>>>(f, la, c.link, c.pm, c.hz, c.prm.thetamaxsqd, daux,
-                                                 c.gA, c.gB, c.gC, c.hA, c.hmax, c.bbmin, c.bbmax,
-                                                 c.info.root[0], c.info.root[1], c.info.root[2],
-                                                 delta, c.nkids, c.wA, c.hA32, c.hN,
-                                                 c.ncloud > 1 ? c.d_clouds : nullptr, c.ncloud);
-    ++c.nlaunch;
+    k_stock_level<<<nb(la - f + 1, 128), 128, 0, c.st>>>(f, la, a); ++c.nlaunch;
   }
+  k_stock_top<<<1, TOP_T, 0, c.st>>>(top, level_first(c, top), a); ++c.nlaunch;
 }
 
 void launch_update_hmax(Ctx& c) {
-  for (int l = c.info.ltot; l >= 0; --l) {
+  const int top = top_levels(c);
+  for (int l = c.info.ltot; l >= top; --l) {
     const int f = c.info.first_cell[l], la = c.info.last_cell[l];
-    const int cnt = la - f + 1;
-    if (cnt <= 0) continue;
-    k_hmax_level<<<nb(cnt, 128), 128, 0, c.st>>>(f, la, c.link, c.hz, c.hrm, c.hrm32, c.hN); ++c.nlaunch;
+    k_hmax_level<<<nb(la - f + 1, 128), 128, 0, c.st>>>(f, la, c.link, c.nkids, c.hz, c.hrm,
+                                                        c.hrm32, c.hN); ++c.nlaunch;
   }
+  k_hmax_top<<<1, TOP_T, 0, c.st>>>(top, level_first(c, top), c.link, c.nkids, c.hz, c.hrm,
+                                    c.hrm32, c.hN); ++c.nlaunch;
 }
 
 void launch_hguess(Ctx& c) {
