@@ -1011,6 +1011,65 @@ __device__ int rd_walk(const HydroTree& t, int root, int lane, int* fa, int* fb,
   return nleaf;
 }
 
+// f(q, pos) for every neighbour q of p as get_neib keeps them (sph/get_neib.F90:83-118: r^2
+// <= 4h_p^2 or r^2 <= 4h_q^2), each on one lane, pos its place in a fixed order, from a
+// gather-or-scatter walk (BHhydro_walk.F90:37-43) through scratch (three buffers
+// of cap entries), SEG leaves at a time through cand, or beyond them the
+// stackless walk of one lane; returns their number.  Every lane takes part.
+template <int SEG, class F>
+__device__ int neib_each(int p, const double4& P, double hp, const double4* __restrict__ pm,
+                         const double2* __restrict__ hz, const HydroTree& t, int* scratch,
+                         int cap, int* cand, int lane, DevError* err, F&& f) {
+  const double hsp = (KERNRANGESQD * hp) * hp;
+  const double R = KERNRANGE * hp;
+  auto test = [&](int c) {
+    const double4 h = t.hA[c];
+    const double d0 = h.x - P.x, d1 = h.y - P.y, d2 = h.z - P.z;
+    const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
+    const double t1 = R + h.w;
+    const double t2 = t.hrm[c] + h.w;
+    return drsqd <= t1 * t1 || drsqd <= t2 * t2;
+  };
+  auto keep = [&](int q) {
+    if (q == p) return false;
+    const double4 Q = pm[q];
+    const double hq = hz[q].x;
+    const double hsq = (KERNRANGESQD * hq) * hq;
+    const double d0 = Q.x - P.x, d1 = Q.y - P.y, d2 = Q.z - P.z;
+    const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
+    return drsqd <= hsp || drsqd <= hsq;
+  };
+  const int root = frame_for(t, p).root;
+  int* fa = scratch;
+  int* lv = scratch + 2 * (size_t)cap;
+  int cnt = 0, kept = 0;
+  unsigned long long nvisit = 0;
+  const int nl = rd_walk(t, root, lane, fa, fa + cap, lv, cap, cnt, nvisit, test);
+  if (nl < 0) {
+    if (lane == 0)
+      walk_gather_scatter(t, root, P.x, P.y, P.z, R, err, p, [&](int q) {
+        if (keep(q)) f(q, kept++);
+      });
+    return __shfl_sync(FULL, kept, 0);
+  }
+  for (int s0 = 0; s0 < nl; s0 += SEG) {
+    const int nc = gp_flatten(lv + s0, min(SEG, nl - s0), cand, lane);
+    int nk = 0;                                      // those kept, packed in place
+    for (int b = 0; b < nc; b += 32) {
+      const int q = b + lane < nc ? cand[b + lane] : p;
+      const bool k = keep(q);
+      const unsigned m = __ballot_sync(FULL, k);
+      if (k) cand[nk + __popc(m & ((1u << lane) - 1u))] = q;
+      nk += __popc(m);
+    }
+    __syncwarp();
+    for (int k = lane; k < nk; k += 32) f(cand[k], kept + k);
+    kept += nk;
+    __syncwarp();
+  }
+  return kept;
+}
+
 __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
     const int* __restrict__ redo, const int* __restrict__ nredo, const double4* __restrict__ pm,
     double2* __restrict__ hz, const double4* __restrict__ vel, double* __restrict__ rho,
@@ -1980,6 +2039,7 @@ __device__ __forceinline__ float m4_w1_bin(float x, bool tc) {
 }
 
 constexpr int HY_SUB = 4;        // threads per particle in the mixed hydro kernel
+constexpr int HY_SUB64 = 8;      // and in the FP64 one (1M core: 1.82 ms with 1, 1.45 with 4 or 8; 777: 132, 52, 39 us)
 
 // SUB consecutive threads share one particle, each taking every SUB-th entry
 // of its neighbour list, and their sums are added at the end (SUB = 1 keeps the
@@ -2008,61 +2068,76 @@ __global__ void k_hydro_prep_pack(int n, const double4* __restrict__ pm,
   rec[3 * (size_t)p + 2] = make_double4(pfv, hfv, sound[p], r);
 }
 
-// PACKED: the neighbours' values come from k_hydro_prep_pack's records (rec), else
-// from the separate arrays (the form without a context keeps those)
-template <bool MIXED, int SUB, bool PACKED = false>
-__global__ void __launch_bounds__(128, 8) k_hydro(int nact, const int* __restrict__ act,
-                                               const double4* __restrict__ pm,
-                                               const double2* __restrict__ hz,
-                                               const double4* __restrict__ vel,
-                                               const double* __restrict__ rho,
-                                               const double* __restrict__ pf,
-                                               const double* __restrict__ hf4,
-                                               const double* __restrict__ sound,
-                                               const int* __restrict__ pptot,
-                                               const int* __restrict__ pplist, int L, HydroTree t,
-                                               const double4* __restrict__ tabG, double alpha,
-                                               bool tc, double* __restrict__ acc,
-                                               double* __restrict__ amap, DevError* err,
-                                               const double4* __restrict__ rec = nullptr) {
-  auto ld_pm = [&](int q) { if constexpr (PACKED) return rec[3 * (size_t)q]; else return pm[q]; };
-  auto ld_h = [&](int q) {
-    if constexpr (PACKED) return rec[3 * (size_t)q + 1].w; else return hz[q].x;
-  };
-  auto ld_v = [&](int q) {
-    if constexpr (PACKED) return rec[3 * (size_t)q + 1]; else return vel[q];
-  };
-  auto ld_pf = [&](int q) { if constexpr (PACKED) return rec[3 * (size_t)q + 2].x; else return pf[q]; };
-  auto ld_hf4 = [&](int q) {
-    if constexpr (PACKED) return rec[3 * (size_t)q + 2].y; else return hf4[q];
-  };
-  auto ld_c = [&](int q) {
-    if constexpr (PACKED) return rec[3 * (size_t)q + 2].z; else return sound[q];
-  };
-  auto ld_rho = [&](int q) {
-    if constexpr (PACKED) return rec[3 * (size_t)q + 2].w; else return rho[q];
-  };
-  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = gi / SUB, sub = gi % SUB;
-  if (SUB == 1 && i >= nact) return;
-  const bool valid = i < nact;
-  const int p = valid ? (act ? act[i] : i) : 0;
-  const double4 P = pm[p];
-  const double hp = hz[p].x;
-  const double invhp = 1.0 / hp;
-  const double hfactor_p = hf4[p];
-  const double4 vp = vel[p];
-  const double sound_p = sound[p];
-  const double rho_p = rho[p];
-  const double pfactor_p = pf[p];
-  const double beta = 2.0 * alpha;
+// The arrays of the hydro kernels.  PACKED: the neighbours' values come from
+// k_hydro_prep_pack's records (rec), else from the separate arrays (the form
+// without a context keeps those).
+struct HydroArrays {
+  const double4* __restrict__ pm;
+  const double2* __restrict__ hz;
+  const double4* __restrict__ vel;
+  const double* __restrict__ rho;
+  const double* __restrict__ pf;
+  const double* __restrict__ hf4;
+  const double* __restrict__ sound;
+  const double4* __restrict__ rec;
+  const double4* __restrict__ tabG;
+  double alpha;
+  bool tc;
+};
+
+// One particle's hydro sums (hydro_gradh.F90:91-297): its own values, and pair(q) adds
+// neighbour q.
+template <bool MIXED, bool PACKED>
+struct HydroSum {
+  const HydroArrays& A;
+  double4 P, vp;
+  double hp, invhp, hfactor_p, sound_p, rho_p, pfactor_p, alpha, beta;
   double at0 = 0.0, at1 = 0.0, at2 = 0.0, ad0 = 0.0, ad1 = 0.0, ad2 = 0.0;
   // FP32 form
-  const float hp32 = (float)hp, invhp32 = (float)invhp, hf32 = (float)hfactor_p;
-  const float pf32 = (float)pfactor_p, c32 = (float)sound_p, rho32 = (float)rho_p;
-  const float alpha32 = (float)alpha, beta32 = (float)beta;
+  float hp32, invhp32, hf32, pf32, c32, rho32, alpha32, beta32;
   float f0 = 0.f, f1 = 0.f, f2 = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f;
-  auto pair = [&](int q) {
+  const double4* tabG;
+  bool tc;
+
+  __device__ __forceinline__ HydroSum(const HydroArrays& a, int p) : A(a) {
+    P = a.pm[p];
+    vp = a.vel[p];
+    hp = a.hz[p].x;
+    invhp = 1.0 / hp;
+    hfactor_p = a.hf4[p];
+    sound_p = a.sound[p];
+    rho_p = a.rho[p];
+    pfactor_p = a.pf[p];
+    alpha = a.alpha;
+    beta = 2.0 * alpha;
+    hp32 = (float)hp; invhp32 = (float)invhp; hf32 = (float)hfactor_p;
+    pf32 = (float)pfactor_p; c32 = (float)sound_p; rho32 = (float)rho_p;
+    alpha32 = (float)alpha; beta32 = (float)beta;
+    tabG = a.tabG;
+    tc = a.tc;
+  }
+  __device__ __forceinline__ double4 ld_pm(int q) const {
+    if constexpr (PACKED) return A.rec[3 * (size_t)q]; else return A.pm[q];
+  }
+  __device__ __forceinline__ double ld_h(int q) const {
+    if constexpr (PACKED) return A.rec[3 * (size_t)q + 1].w; else return A.hz[q].x;
+  }
+  __device__ __forceinline__ double4 ld_v(int q) const {
+    if constexpr (PACKED) return A.rec[3 * (size_t)q + 1]; else return A.vel[q];
+  }
+  __device__ __forceinline__ double ld_pf(int q) const {
+    if constexpr (PACKED) return A.rec[3 * (size_t)q + 2].x; else return A.pf[q];
+  }
+  __device__ __forceinline__ double ld_hf4(int q) const {
+    if constexpr (PACKED) return A.rec[3 * (size_t)q + 2].y; else return A.hf4[q];
+  }
+  __device__ __forceinline__ double ld_c(int q) const {
+    if constexpr (PACKED) return A.rec[3 * (size_t)q + 2].z; else return A.sound[q];
+  }
+  __device__ __forceinline__ double ld_rho(int q) const {
+    if constexpr (PACKED) return A.rec[3 * (size_t)q + 2].w; else return A.rho[q];
+  }
+  __device__ __forceinline__ void pair(int q) {
     const double4 Q = ld_pm(q);
     const double hq = ld_h(q);
     if (MIXED) {
@@ -2139,54 +2214,102 @@ __global__ void __launch_bounds__(128, 8) k_hydro(int nact, const int* __restric
       ad1 = ad1 - ((g * u1) * wmean) / rhomean;
       ad2 = ad2 - ((g * u2) * wmean) / rhomean;
     }
-  };
+  }
+  // the sums over n consecutive lanes (a power of two)
+  __device__ __forceinline__ void reduce(int n) {
+    for (int o = n / 2; o > 0; o >>= 1) {
+      if constexpr (MIXED) {
+        f0 += __shfl_xor_sync(FULL, f0, o);
+        f1 += __shfl_xor_sync(FULL, f1, o);
+        f2 += __shfl_xor_sync(FULL, f2, o);
+        g0 += __shfl_xor_sync(FULL, g0, o);
+        g1 += __shfl_xor_sync(FULL, g1, o);
+        g2 += __shfl_xor_sync(FULL, g2, o);
+      } else {
+        at0 += __shfl_xor_sync(FULL, at0, o);
+        at1 += __shfl_xor_sync(FULL, at1, o);
+        at2 += __shfl_xor_sync(FULL, at2, o);
+        ad0 += __shfl_xor_sync(FULL, ad0, o);
+        ad1 += __shfl_xor_sync(FULL, ad1, o);
+        ad2 += __shfl_xor_sync(FULL, ad2, o);
+      }
+    }
+  }
+  // the acceleration to acc and, when given, to a mapped host buffer (straight
+  // over PCIe)
+  __device__ __forceinline__ void store(int p, double* __restrict__ acc,
+                                        double* __restrict__ amap) const {
+    double r0, r1, r2;
+    if constexpr (MIXED) {
+      r0 = (double)f0 + (double)g0;
+      r1 = (double)f1 + (double)g1;
+      r2 = (double)f2 + (double)g2;
+    } else {
+      r0 = at0 + ad0;                                                            // :287, :297
+      r1 = at1 + ad1;
+      r2 = at2 + ad2;
+    }
+    double* a = acc + (size_t)p * 3;
+    a[0] = r0;
+    a[1] = r1;
+    a[2] = r2;
+    if (amap) {
+      amap[(size_t)p * 3] = r0;
+      amap[(size_t)p * 3 + 1] = r1;
+      amap[(size_t)p * 3 + 2] = r2;
+    }
+  }
+};
+
+// A particle whose neighbours outnumber its list (pptot > pp_limit) goes to over /
+// nover, for k_hydro_over; without them (the form without a context) there is none.
+template <bool MIXED, int SUB, bool PACKED = false>
+__global__ void __launch_bounds__(128, 8) k_hydro(int nact, const int* __restrict__ act,
+                                               HydroArrays A, const int* __restrict__ pptot,
+                                               const int* __restrict__ pplist, int L,
+                                               double* __restrict__ acc, double* __restrict__ amap,
+                                               int* __restrict__ over, int* __restrict__ nover) {
+  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = gi / SUB, sub = gi % SUB;
+  const bool valid = i < nact;
+  const int p = valid ? (act ? act[i] : i) : 0;
+  HydroSum<MIXED, PACKED> H(A, p);
   const int nn = valid ? pptot[p] : 0;
   if (nn <= L) {
     const int* row = pplist + (size_t)p * L;
-    for (int k = sub; k < nn; k += SUB) pair(row[k]);
-  } else if (sub == 0) {
-    // get_neib_on_fly (sph/get_neib_on_fly.F90:11-130): same test as get_neib
-    const double hsp = (KERNRANGESQD * hp) * hp;
-    walk_gather_scatter(t, frame_for(t, p).root, P.x, P.y, P.z, KERNRANGE * hp, err, p, [&](int q) {
-      if (q == p) return;
-      const double hq = ld_h(q);
-      const double hsq = (KERNRANGESQD * hq) * hq;
-      const double4 Q = ld_pm(q);
-      const double d0 = Q.x - P.x, d1 = Q.y - P.y, d2 = Q.z - P.z;
-      const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
-      if (drsqd <= hsp || drsqd <= hsq) pair(q);
-    });
+    for (int k = sub; k < nn; k += SUB) H.pair(row[k]);
+  } else if (sub == 0 && over) {
+    over[atomicAdd(nover, 1)] = p;
   }
-  if (SUB > 1) {
-#pragma unroll
-    for (int o = SUB / 2; o > 0; o >>= 1) {
-      f0 += __shfl_xor_sync(0xffffffffu, f0, o);
-      f1 += __shfl_xor_sync(0xffffffffu, f1, o);
-      f2 += __shfl_xor_sync(0xffffffffu, f2, o);
-      g0 += __shfl_xor_sync(0xffffffffu, g0, o);
-      g1 += __shfl_xor_sync(0xffffffffu, g1, o);
-      g2 += __shfl_xor_sync(0xffffffffu, g2, o);
-    }
-    if (!valid || sub != 0) return;
-  }
-  double r0, r1, r2;
-  if (MIXED) {
-    r0 = (double)f0 + (double)g0;
-    r1 = (double)f1 + (double)g1;
-    r2 = (double)f2 + (double)g2;
-  } else {
-    r0 = at0 + ad0;                                                              // :287, :297
-    r1 = at1 + ad1;
-    r2 = at2 + ad2;
-  }
-  double* a = acc + (size_t)p * 3;
-  a[0] = r0;
-  a[1] = r1;
-  a[2] = r2;
-  if (amap) {                                  // a mapped host buffer: straight over PCIe
-    amap[(size_t)p * 3] = r0;
-    amap[(size_t)p * 3 + 1] = r1;
-    amap[(size_t)p * 3 + 2] = r2;
+  __syncwarp();
+  H.reduce(SUB);
+  if (valid && sub == 0 && nn <= L) H.store(p, acc, amap);
+}
+
+// The particles k_hydro left: one warp each, the neighbours from a walk
+// (get_neib_on_fly, sph/get_neib_on_fly.F90:11-130: the same test as get_neib) spread
+// over the lanes, breadth first through the redo kernel's scratch; a walk
+// beyond it falls back to the stackless walk of one lane.  (One thread walking
+// alone took 0.3 ms of the hydro kernel of a 50000-particle disc.)
+template <bool MIXED, bool PACKED>
+__global__ void __launch_bounds__(RD_THREADS) k_hydro_over(
+    const int* __restrict__ over, const int* __restrict__ nover, HydroArrays A, HydroTree t,
+    int* __restrict__ scratch, int cap, double* __restrict__ acc, double* __restrict__ amap,
+    DevError* err) {
+  __shared__ int cand_all[RD_WARPS][GP_SEG * LEAFMAX];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int gw = blockIdx.x * RD_WARPS + w;
+  const int n = *nover;
+  for (int i = gw; i < n; i += gridDim.x * RD_WARPS) {
+    const int p = over[i];
+    HydroSum<MIXED, PACKED> H(A, p);
+    const double4 P = A.pm[p];
+    const double hp = A.hz[p].x;
+    neib_each<GP_SEG>(p, P, hp, A.pm, A.hz, t, scratch + (size_t)gw * 3 * cap, cap, cand_all[w], lane, err,
+              [&](int q, int) { H.pair(q); });
+    __syncwarp();
+    H.reduce(32);
+    if (lane == 0) H.store(p, acc, amap);
   }
 }
 
@@ -2442,75 +2565,6 @@ void launch_neib(Ctx& c, int nact, bool sorted) {
 //    to run: the gather part in the final pass's order, then the scatter part).
 // pptot ends as the full count in every row (the reference's pp_tot), and a
 // row of more than pp_limit neighbours keeps no list, as in the reference.
-__global__ void k_neib_flag(int n, const int* __restrict__ npot, int* __restrict__ flag) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < n) flag[p] = npot[p] < 0 ? 1 : 0;
-}
-
-__global__ void k_neib_list(int n, const int* __restrict__ flag, const int* __restrict__ scan,
-                            int* __restrict__ out) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < n && flag[p]) out[scan[p]] = p;
-}
-
-// position and h of every particle, h negated for a walked row (npot = -1),
-// so that the transposition gathers one 32-byte record per neighbour
-__global__ void k_neib_hflag(int n, const double4* __restrict__ pm, const double2* __restrict__ hz,
-                             const int* __restrict__ npot, double4* __restrict__ ph) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const double4 P = pm[p];
-  const double h = hz[p].x;
-  ph[p] = make_double4(P.x, P.y, P.z, npot[p] < 0 ? -h : h);
-}
-
-// one warp per particle p: its gather neighbours q, from its row (the first
-// npot[p] entries; the gather part of a walked row), or from a walk when the
-// row has more than L; p joins q's row when q's own gather set lacks it
-constexpr int NT_THREADS = 256;
-__global__ void __launch_bounds__(NT_THREADS) k_neib_transpose(
-    int n, const double4* __restrict__ ph, const int* __restrict__ npot, int* __restrict__ pptot,
-    int* __restrict__ pplist, int L, HydroTree t, DevError* err, unsigned long long* counts) {
-  const int lane = threadIdx.x & 31;
-  const int nw = gridDim.x * (NT_THREADS / 32);
-  unsigned long long ntest = 0;
-  for (int p = blockIdx.x * (NT_THREADS / 32) + (threadIdx.x >> 5); p < n; p += nw) {
-    const int g0 = npot[p];
-    // a walked row is complete and final; a recorded row grows from g0 on
-    const int ng = g0 >= 0 ? g0 : pptot[p];
-    const double4 P = ph[p];
-    const double hp = fabs(P.w);
-    const double hsp = (KERNRANGESQD * hp) * hp;
-    auto visit = [&](int q, bool test_gather) {
-      const double4 Q = ph[q];
-      const double hq = Q.w;
-      const double d0 = Q.x - P.x, d1 = Q.y - P.y, d2 = Q.z - P.z;
-      const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
-      if (test_gather && !(drsqd <= hsp)) return;
-      if (hq < 0.0) return;                          // q's row came from a walk
-      if (drsqd <= (KERNRANGESQD * hq) * hq) return; // p is in q's gather set
-      const int slot = atomicAdd(pptot + q, 1);
-      if (slot < L) pplist[(size_t)q * L + slot] = p;
-    };
-    if (ng <= L) {
-      const int* row = pplist + (size_t)p * L;
-      for (int k = lane; k < ng; k += 64) {          // two entries per lane in flight
-        const int q0 = row[k];
-        const int q1 = k + 32 < ng ? row[k + 32] : -1;
-        visit(q0, g0 < 0);
-        if (q1 >= 0) visit(q1, g0 < 0);
-      }
-      ntest += ng;
-    } else if (lane == 0) {                          // more than L: the gather set from a walk
-      walk_gather_scatter(t, frame_for(t, p).root, P.x, P.y, P.z, KERNRANGE * hp, err, p,
-                          [&](int q) {
-                            if (q != p) visit(q, true);
-                          });
-    }
-  }
-  if (lane == 0) atomicAdd(counts + 7, ntest);
-}
-
 // bitonic sort of N = 32 R values per warp, value r*32 + lane in e[r] (or,
 // with R = 1, of the first N <= 32 lanes' values, each block of N lanes on
 // its own, the first one ascending)
@@ -2562,134 +2616,214 @@ __device__ __forceinline__ void sort_row(int* row, int m, int lane) {
   }
 }
 
-// one warp per recorded row that holds its whole list: the row in increasing
-// order (full), or only its scatter part (the entries the transposition
-// appended, in an order that depends on the atomics), so that the row's order
-// is the same from run to run
-__global__ void __launch_bounds__(NT_THREADS) k_neib_sort(int n, const int* __restrict__ npot,
-                                                         const int* __restrict__ pptot,
-                                                         int* __restrict__ pplist, int L,
-                                                         int full) {
-  const int lane = threadIdx.x & 31;
-  const int nw = gridDim.x * (NT_THREADS / 32);
-  for (int p = blockIdx.x * (NT_THREADS / 32) + (threadIdx.x >> 5); p < n; p += nw) {
-    const int g0 = npot[p];
-    if (g0 < 0) continue;                            // a walked row: in order already
-    const int tot = pptot[p];
-    if (tot > L) continue;
-    const int b = full ? 0 : g0;
-    const int m = tot - b;
-    if (m < 2) continue;
-    int* row = pplist + (size_t)p * L + b;
-    if (m <= 8) sort_row<1, 8>(row, m, lane);
-    else if (m <= 16) sort_row<1, 16>(row, m, lane);
-    else if (m <= 32) sort_row<1>(row, m, lane);
-    else if (m <= 64) sort_row<2>(row, m, lane);
-    else if (m <= 128) sort_row<4>(row, m, lane);
-    else if (m <= 256) sort_row<8>(row, m, lane);
-    else if (lane == 0) {                            // pp_limit above 256: insertion sort
-      for (int i = 1; i < m; ++i) {
-        const int x = row[i];
-        int j = i - 1;
-        while (j >= 0 && row[j] > x) {
-          row[j + 1] = row[j];
-          --j;
+// a row of m values in increasing order, by one warp
+__device__ __forceinline__ void sort_any(int* row, int m, int lane) {
+  if (m < 2) return;
+  if (m <= 32) sort_row<1>(row, m, lane);
+  else if (m <= 64) sort_row<2>(row, m, lane);
+  else if (m <= 128) sort_row<4>(row, m, lane);
+  else if (m <= 256) sort_row<8>(row, m, lane);
+  else if (lane == 0) {                              // pp_limit above 256: insertion sort
+    for (int i = 1; i < m; ++i) {
+      const int x = row[i];
+      int j = i - 1;
+      while (j >= 0 && row[j] > x) {
+        row[j + 1] = row[j];
+        --j;
+      }
+      row[j + 1] = x;
+    }
+  }
+}
+
+// ascending bitonic sort of 16 values over 8 lanes, value r*8 + l8 in e[r]
+__device__ __forceinline__ void oct_bitonic(int (&e)[2], int l8) {
+#pragma unroll
+  for (int size = 2; size <= 16; size <<= 1) {
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      if (stride == 8) {                             // (size 16: ascending)
+        const int a = min(e[0], e[1]), b = max(e[0], e[1]);
+        e[0] = a;
+        e[1] = b;
+      } else {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const bool up = ((r * 8 + l8) & size) == 0;
+          const int o = __shfl_xor_sync(FULL, e[r], stride);
+          const bool lower = (l8 & stride) == 0;
+          e[r] = (lower == up) ? min(e[r], o) : max(e[r], o);
         }
-        row[j + 1] = x;
       }
     }
+  }
+}
+
+// k_neib_hflag writes what the transposition gathers of a neighbour, one 16-byte
+// record (FP32 position relative to the particle's root centre, h rounded; h
+// negated for a walked row), half the bytes of FP64, and lists the particles that
+// need a walk: the rows to walk, and recorded rows with more than L gather
+// neighbours.
+__global__ void k_neib_hflag(int n, const double4* __restrict__ pm, const double2* __restrict__ hz,
+                             const int* __restrict__ npot, int L, HydroTree t,
+                             float4* __restrict__ ph, int* __restrict__ list,
+                             int* __restrict__ nlist) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  bool walk = false;
+  if (p < n) {
+    const TreeFrame fr = frame_for(t, p);
+    const double4 P = pm[p];
+    const float h = (float)hz[p].x;
+    const int g0 = npot[p];
+    walk = g0 < 0 || g0 > L;
+    ph[p] = make_float4((float)(P.x - fr.rootx), (float)(P.y - fr.rooty), (float)(P.z - fr.rootz),
+                        g0 < 0 ? -h : h);
+  }
+  const unsigned b = __ballot_sync(FULL, walk);
+  if (b != 0u) {
+    const int lane = threadIdx.x & 31;
+    int o = 0;
+    if (lane == 0) o = atomicAdd(nlist, __popc(b));
+    o = __shfl_sync(FULL, o, 0);
+    if (walk) list[o + __popc(b & ((1u << lane) - 1u))] = p;
+  }
+}
+
+// neighbour q of p (record G) in the transposition: p joins q's row when q's own
+// gather set lacks it (r^2 > 4h_q^2; q's row recorded, not walked); test_gather: only
+// when q is a gather neighbour of p at all.  FP32 decides away from the bounds
+// (test32), the FP64 values otherwise.
+__device__ __forceinline__ void neib_visit(int p, int q, const float4& F, const float4& G,
+                                           float delta, bool test_gather,
+                                           const double4* __restrict__ pm,
+                                           const double2* __restrict__ hz, int* __restrict__ pptot,
+                                           int* __restrict__ pplist, int L) {
+  if (G.w < 0.0f) return;                          // q's row comes from a walk
+  const float e0 = G.x - F.x, e1 = G.y - F.y, e2 = G.z - F.z;
+  const float r2 = (e0 * e0 + e1 * e1) + e2 * e2;
+  const int in_q = test32(r2, 2.0f * G.w, delta);  // p in q's gather set
+  if (in_q == 1) return;
+  const int in_p = test_gather ? test32(r2, 2.0f * fabsf(F.w), delta) : 1;
+  if (in_p == 0) return;
+  if (in_q < 0 || in_p < 0) {
+    const double4 P = pm[p], Q = pm[q];
+    const double hp = hz[p].x, hq = hz[q].x;
+    const double d0 = Q.x - P.x, d1 = Q.y - P.y, d2 = Q.z - P.z;
+    const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
+    if (drsqd <= (KERNRANGESQD * hq) * hq) return;
+    if (test_gather && !(drsqd <= (KERNRANGESQD * hp) * hp)) return;
+  }
+  const int slot = atomicAdd(pptot + q, 1);
+  if (slot < L) pplist[(size_t)q * L + slot] = p;
+}
+
+// Blocks from wblocks on: one warp per particle p with a recorded row of at most L,
+// its gather neighbours q the first npot[p] entries.  The first wblocks blocks: one
+// warp per listed particle (k_neib_hflag), its neighbours from a walk; for a walked
+// row they are its list, kept as get_neib keeps them (sph/get_neib.F90:83-118) and
+// put in increasing order.  Neither reads what the other writes: a walked row
+// takes no scatter entries.  (As kernels of their own, the few walks were 50 us of
+// latency each.)  Bound by the latency of the record gathers, so 8 blocks per SM: 4M
+// core 1.67 ms, 2.02 at 6, 1.97 with FP64 records of 32 bytes.
+constexpr int NT_THREADS = 256;
+constexpr int NT_WARPS = NT_THREADS / 32;
+constexpr int NT_SEG = 8;        // (little shared memory: the gathers live on L1)
+__global__ void __launch_bounds__(NT_THREADS, 8) k_neib_transpose(
+    int n, int wblocks, const float4* __restrict__ ph, const double4* __restrict__ pm,
+    const double2* __restrict__ hz, const int* __restrict__ npot, int* __restrict__ pptot,
+    int* __restrict__ pplist, int L, HydroTree t, const int* __restrict__ list,
+    const int* __restrict__ nlist, int* __restrict__ scratch, int cap, DevError* err,
+    unsigned long long* counts) {
+  __shared__ int cand_all[NT_WARPS][NT_SEG * LEAFMAX];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned long long ntest = 0;
+  if (blockIdx.x < wblocks) {
+    const int gw = blockIdx.x * NT_WARPS + w;
+    const int nl = *nlist;
+    for (int i = gw; i < nl; i += wblocks * NT_WARPS) {
+      const int p = list[i];
+      const bool walked = npot[p] < 0;
+      const float4 F = ph[p];
+      const float delta = frame_for(t, p).delta;
+      int* row = pplist + (size_t)p * L;
+      const int kept = neib_each<NT_SEG>(p, pm[p], hz[p].x, pm, hz, t, scratch + (size_t)gw * 3 * cap, cap,
+                                 cand_all[w], lane, err, [&](int q, int pos) {
+        if (walked && pos < L) row[pos] = q;
+        neib_visit(p, q, F, ph[q], delta, true, pm, hz, pptot, pplist, L);
+      });
+      ntest += kept;
+      if (walked) {
+        if (lane == 0) pptot[p] = kept;
+        __syncwarp();
+        if (kept <= L) sort_any(row, kept, lane);
+      }
+      __syncwarp();
+    }
+  } else {
+    const int nw = (gridDim.x - wblocks) * NT_WARPS;
+    for (int p = (blockIdx.x - wblocks) * NT_WARPS + w; p < n; p += nw) {
+      const int ng = npot[p];
+      if (ng < 0 || ng > L) continue;
+      const float4 F = ph[p];
+      const float delta = frame_for(t, p).delta;
+      const int* row = pplist + (size_t)p * L;
+      for (int k = lane; k < ng; k += 64) {          // two entries per lane in flight
+        const int q0 = row[k];
+        const int q1 = k + 32 < ng ? row[k + 32] : q0;
+        const float4 G0 = ph[q0], G1 = ph[q1];
+        neib_visit(p, q0, F, G0, delta, false, pm, hz, pptot, pplist, L);
+        if (k + 32 < ng) neib_visit(p, q1, F, G1, delta, false, pm, hz, pptot, pplist, L);
+      }
+      ntest += ng;
+    }
+  }
+  if (lane == 0) atomicAdd(counts + 7, ntest);
+}
+
+// one warp per recorded row that holds its whole list: the row in increasing order
+__global__ void __launch_bounds__(NT_THREADS) k_neib_sort(int n, const int* __restrict__ npot,
+                                                         const int* __restrict__ pptot,
+                                                         int* __restrict__ pplist, int L) {
+  const int lane = threadIdx.x & 31;
+  const int nw = gridDim.x * NT_WARPS;
+  for (int p = blockIdx.x * NT_WARPS + (threadIdx.x >> 5); p < n; p += nw) {
+    const int tot = pptot[p];
+    if (npot[p] < 0 || tot > L) continue;            // (a walked row is in order already)
+    sort_any(pplist + (size_t)p * L, tot, lane);
     __syncwarp();
   }
 }
 
-// The rows of the particles grad-h left to a walk (npot = -1: redone, or
-// h >= h_high at the final pass): one warp per particle, the reference's
-// gather-or-scatter walk (BHhydro_walk.F90:37-43, FP64 test) breadth first
-// through the redo kernel's scratch, the neighbours kept as get_neib keeps
-// them (sph/get_neib.F90:83-118) and put in increasing order; a walk beyond
-// the scratch falls back to the stackless walk of one thread.
-__global__ void __launch_bounds__(RD_THREADS) k_neib_walked(
-    int nw, const int* __restrict__ list, const double4* __restrict__ pm,
-    const double2* __restrict__ hz, HydroTree t, int L, int* __restrict__ pptot,
-    int* __restrict__ pplist, int* __restrict__ scratch, int cap, DevError* err,
-    unsigned long long* counts) {
-  __shared__ int cand_all[RD_WARPS][GP_SEG * LEAFMAX];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int* cand = cand_all[w];
-  const int gw = blockIdx.x * RD_WARPS + w;
-  int* fa = scratch + (size_t)gw * 3 * cap;
-  int* fb = fa + cap;
-  int* lv = fb + cap;
-  const unsigned lt = (1u << lane) - 1u;
-  unsigned long long nvisit = 0, ncands = 0;
-  for (int i = gw; i < nw; i += gridDim.x * RD_WARPS) {
-    const int p = list[i];
-    const double4 P = pm[p];
-    const double hp = hz[p].x;
-    const double hsp = (KERNRANGESQD * hp) * hp;
-    const double R = KERNRANGE * hp;
-    auto test = [&](int c) {
-      const double4 h = t.hA[c];
-      const double d0 = h.x - P.x, d1 = h.y - P.y, d2 = h.z - P.z;
-      const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
-      const double t1 = R + h.w;
-      const double t2 = t.hrm[c] + h.w;
-      return drsqd <= t1 * t1 || drsqd <= t2 * t2;
-    };
-    int cnt = 0;
-    const int nl = rd_walk(t, frame_for(t, p).root, lane, fa, fb, lv, cap, cnt, nvisit, test);
-    if (nl < 0) {
-      if (lane == 0) neib_one(p, pm, hz, t, L, pptot, pplist, err);
-      __syncwarp();
-      continue;
+// Only the scatter parts of those rows (the entries the transposition appended, in
+// an order that depends on the atomics), so that a row's order is the same
+// from run to run: four rows per warp, eight lanes each, up to 16 entries; a
+// longer part by the whole warp.  (4M core: 0.41 ms; 0.90 with a warp per row.)
+__global__ void __launch_bounds__(NT_THREADS) k_neib_sort8(int n, const int* __restrict__ npot,
+                                                          const int* __restrict__ pptot,
+                                                          int* __restrict__ pplist, int L) {
+  const int lane = threadIdx.x & 31, l8 = lane & 7;
+  const int p = (blockIdx.x * NT_THREADS + threadIdx.x) >> 3;
+  int m = 0;
+  int* row = nullptr;
+  if (p < n) {
+    const int g0 = npot[p], tot = pptot[p];
+    if (g0 >= 0 && tot <= L) {
+      m = tot - g0;
+      row = pplist + (size_t)p * L + g0;
     }
-    int* row = pplist + (size_t)p * L;
-    int kept = 0;
-    for (int s0 = 0; s0 < nl; s0 += GP_SEG) {
-      const int nc = gp_flatten(lv + s0, min(GP_SEG, nl - s0), cand, lane);
-      for (int b = 0; b < nc; b += 32) {
-        const int k = b + lane;
-        const int q = k < nc ? cand[k] : p;
-        bool keep = false;
-        if (q != p) {
-          const double4 Q = pm[q];
-          const double hq = hz[q].x;
-          const double hsq = (KERNRANGESQD * hq) * hq;
-          const double d0 = Q.x - P.x, d1 = Q.y - P.y, d2 = Q.z - P.z;
-          const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
-          keep = drsqd <= hsp || drsqd <= hsq;
-        }
-        const unsigned m = __ballot_sync(FULL, keep);
-        const int pos = kept + __popc(m & lt);
-        if (keep && pos < L) row[pos] = q;
-        kept += __popc(m);
-      }
-      ncands += nc;
-    }
-    if (lane == 0) pptot[p] = kept;
-    __syncwarp();
-    if (kept <= L && kept >= 2) {
-      if (kept <= 32) sort_row<1>(row, kept, lane);
-      else if (kept <= 64) sort_row<2>(row, kept, lane);
-      else if (kept <= 128) sort_row<4>(row, kept, lane);
-      else if (kept <= 256) sort_row<8>(row, kept, lane);
-      else if (lane == 0) {
-        for (int a = 1; a < kept; ++a) {
-          const int x = row[a];
-          int j = a - 1;
-          while (j >= 0 && row[j] > x) {
-            row[j + 1] = row[j];
-            --j;
-          }
-          row[j + 1] = x;
-        }
-      }
-    }
-    __syncwarp();
   }
-  if (lane == 0) {
-    atomicAdd(counts + 4, nvisit);
-    atomicAdd(counts + 7, ncands);
+  const bool few = m <= 16;
+  int e[2];
+  e[0] = few && l8 < m ? row[l8] : INT_MAX;
+  e[1] = few && l8 + 8 < m ? row[l8 + 8] : INT_MAX;
+  oct_bitonic(e, l8);
+  if (few && l8 < m) row[l8] = e[0];
+  if (few && l8 + 8 < m) row[l8 + 8] = e[1];
+  for (unsigned b = __ballot_sync(FULL, !few && l8 == 0); b != 0u; b &= b - 1u) {
+    const int src = __ffs(b) - 1;
+    const int pj = __shfl_sync(FULL, p, src), mj = __shfl_sync(FULL, m, src);
+    sort_any(pplist + (size_t)pj * L + npot[pj], mj, lane);
+    __syncwarp();
   }
 }
 
@@ -2698,31 +2832,24 @@ static void launch_neib_gsets(Ctx& c, bool sorted) {
   const HydroTree t = hydro_tree(c);
   const int n = c.ptot;
   const int L = c.prm.pp_limit;
-  // the particles grad-h left to a walk, in order (c.redo is free after grad-h)
-  k_neib_flag<<<nb(n, 256), 256, 0, c.st>>>(n, c.npot, c.bflag);
-  scan_exclusive(c, c.bflag, c.bscan, n);
-  k_neib_list<<<nb(n, 256), 256, 0, c.st>>>(n, c.bflag, c.bscan, c.redo);
-  c.nlaunch += 2;
-  int nw = 0;
-  read_dev(c, c.scan.total, &nw, sizeof(int));
-  if (nw > 0) {
-    // three walk-stack slots of scratch per warp, as the redo kernel
-    const int blocks = std::min((c.wstack_slots / 3) / RD_WARPS, nb(nw, RD_WARPS));
-    k_neib_walked<<<std::max(1, blocks), RD_THREADS, 0, c.st>>>(
-        nw, c.redo, c.pm, c.hz, t, L, c.pptot, c.pplist, reinterpret_cast<int*>(c.wstack),
-        2 * c.wstack_cap, c.d_err, counts);
-    ++c.nlaunch;
-  }
-  // positions with h and the walked flag, one record per particle, in the
-  // pm_alt reorder target (free between reorders: the next one overwrites it)
-  double4* ph = c.pm_alt;
-  k_neib_hflag<<<nb(n, 256), 256, 0, c.st>>>(n, c.pm, c.hz, c.npot, ph);
+  // the transposition's records, in the pm_alt reorder target (free between
+  // reorders: the next one overwrites it), and the particles that need a walk, in
+  // c.redo (free after grad-h)
+  cudaMemsetAsync(c.work + 1, 0, sizeof(int), c.st);
+  float4* ph = reinterpret_cast<float4*>(c.pm_alt);
+  k_neib_hflag<<<nb(n, 256), 256, 0, c.st>>>(n, c.pm, c.hz, c.npot, L, t, ph, c.redo, c.work + 1);
+  // three walk-stack slots of scratch per warp, as the redo kernel
+  const int wblocks = std::max(1, (c.wstack_slots / 3) / NT_WARPS);
   const int blocks = std::min(sm_count(c) * 8, nb((long)n * 32, NT_THREADS));
-  k_neib_transpose<<<blocks, NT_THREADS, 0, c.st>>>(n, ph, c.npot, c.pptot, c.pplist, L, t,
-                                                    c.d_err, counts);
-  ++c.nlaunch;
-  k_neib_sort<<<blocks, NT_THREADS, 0, c.st>>>(n, c.npot, c.pptot, c.pplist, L, sorted ? 1 : 0);
-  c.nlaunch += 2;
+  k_neib_transpose<<<wblocks + blocks, NT_THREADS, 0, c.st>>>(
+      n, wblocks, ph, c.pm, c.hz, c.npot, c.pptot, c.pplist, L, t, c.redo, c.work + 1,
+      reinterpret_cast<int*>(c.wstack), 2 * c.wstack_cap, c.d_err, counts);
+  if (sorted)
+    k_neib_sort<<<blocks, NT_THREADS, 0, c.st>>>(n, c.npot, c.pptot, c.pplist, L);
+  else
+    k_neib_sort8<<<nb((long)n * 8, NT_THREADS), NT_THREADS, 0, c.st>>>(n, c.npot, c.pptot,
+                                                                        c.pplist, L);
+  c.nlaunch += 3;
 }
 
 int hydro_records(Ctx& c) {
@@ -2745,21 +2872,29 @@ void launch_hydro(Ctx& c, int nact, double* amap) {
     k_hydro_prep<<<nb(c.ptot, 256), 256, 0, c.st>>>(c.ptot, c.hz, c.rho, c.omega, c.press, c.pf,
                                                     c.hf4);
   ++c.nlaunch;
-  const HydroTree t = hydro_tree(c);
-  const bool tc = c.prm.kernel == 1;
+  const HydroArrays A{c.pm, c.hz, c.vel, c.rho, c.pf, c.hf4, c.sound, c.hrec, c.tabG, c.prm.alpha,
+                      c.prm.kernel == 1};
+  // the overflowed rows are listed in c.redo (free after the neighbour lists)
+  cudaMemsetAsync(c.work + 2, 0, sizeof(int), c.st);
   auto go = [&](auto kern, int sub) {
-    kern<<<nb((long)nact * sub, 128), 128, 0, c.st>>>(
-        nact, c.act, c.pm, c.hz, c.vel, c.rho, c.pf, c.hf4, c.sound, c.pptot, c.pplist,
-        c.prm.pp_limit, t, c.tabG, c.prm.alpha, tc, c.acc, amap, c.d_err, c.hrec);
+    kern<<<nb((long)nact * sub, 128), 128, 0, c.st>>>(nact, c.act, A, c.pptot, c.pplist,
+                                                      c.prm.pp_limit, c.acc, amap, c.redo,
+                                                      c.work + 2);
   };
-  // the records pay for the mixed kernel's threads; the FP64 kernel (one
-  // thread per particle) runs faster on the separate arrays (6.9 against 7.4 ms
-  // on the 4M core)
-  if (c.prm.precision == 0) go(k_hydro<false, 1, false>, 1);
+  // the records pay for the mixed kernel's threads; the FP64 kernel runs faster
+  // on the separate arrays (6.9 against 7.4 ms on the 4M core)
+  if (c.prm.precision == 0) go(k_hydro<false, HY_SUB64, false>, HY_SUB64);
   else if (c.tune.hydro_sub == 2) go(k_hydro<true, 2, true>, 2);
   else if (c.tune.hydro_sub == 8) go(k_hydro<true, 8, true>, 8);
   else go(k_hydro<true, HY_SUB, true>, HY_SUB);
-  ++c.nlaunch;
+  auto over = [&](auto kern) {
+    kern<<<std::max(1, (c.wstack_slots / 3) / RD_WARPS), RD_THREADS, 0, c.st>>>(
+        c.redo, c.work + 2, A, hydro_tree(c), reinterpret_cast<int*>(c.wstack), 2 * c.wstack_cap,
+        c.acc, amap, c.d_err);
+  };
+  if (c.prm.precision == 0) over(k_hydro_over<false, false>);
+  else over(k_hydro_over<true, true>);
+  c.nlaunch += 2;
 }
 
 void launch_hgather(Ctx& c, int nact) {
@@ -2946,18 +3081,17 @@ extern "C" int seren_gpu_hydro_forces_noalloc(int32_t n, const double* parray, c
   if (noalloc_launch(k_hydro_prep, nb(n, 256), 256, st, n, hz, rho, omega, press, pf, hf4) !=
       cudaSuccess)
     return SEREN_GPU_ERR_CUDA;
-  const HydroTree none{};   // every row fits its list, so the kernel never walks a tree
   const int* no_act = nullptr;
   double* no_map = nullptr;
-  const double4* no_rec = nullptr;   // the separate arrays, not packed records
+  int* no_over = nullptr;            // every row fits its list: no walks
+  const HydroArrays A{pm, hz, vel, rho, pf, hf4, sound, nullptr, tab, alpha, kernel == 1};
   const cudaError_t lrc =
-      precision == 0
-          ? noalloc_launch(k_hydro<false, 1>, nb(n, 128), 128, st, n, no_act, pm, hz, vel, rho,
-                           pf, hf4, sound, pptot, pplist, pp_limit, none, tab, alpha,
-                           kernel == 1, a, no_map, d_err, no_rec)
-          : noalloc_launch(k_hydro<true, HY_SUB>, nb((long)n * HY_SUB, 128), 128, st, n, no_act,
-                           pm, hz, vel, rho, pf, hf4, sound, pptot, pplist, pp_limit, none, tab,
-                           alpha, kernel == 1, a, no_map, d_err, no_rec);
+      precision == 0 ? noalloc_launch(k_hydro<false, HY_SUB64>, nb((long)n * HY_SUB64, 128), 128,
+                                      st, n, no_act, A, pptot, pplist, pp_limit, a, no_map,
+                                      no_over, no_over)
+                     : noalloc_launch(k_hydro<true, HY_SUB>, nb((long)n * HY_SUB, 128), 128, st, n,
+                                      no_act, A, pptot, pplist, pp_limit, a, no_map, no_over,
+                                      no_over);
   if (lrc != cudaSuccess) return SEREN_GPU_ERR_CUDA;
   return noalloc_status(st, d_err);
 }
