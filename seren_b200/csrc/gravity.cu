@@ -26,6 +26,7 @@ struct GravTree {
   const double4* gA;   // COM, m
   const double4* gB;   // q1..q4
   const double2* gC;   // q5, dminsqd
+  const int* nkids;    // children per cell
   int ctot;
 };
 
@@ -959,55 +960,95 @@ k_grav_walk(int nact, const int* __restrict__ act, int ngroups, const int* __res
 
 
 // sph_sim/sph_sink_forces.F90:49-110: BHgrav_accel(-s) with gravity_meanh
-// near field (BHgrav_accel.F90:299-314), then the other sinks directly.
-__global__ void k_sink_walk(int nsink, const double* __restrict__ sinks, const double4* __restrict__ pm,
-                            const double2* __restrict__ hz, GravTree t,
-                            const double4* __restrict__ tabG, double* __restrict__ out,
-                            DevError* err) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsink) return;
+// near field (BHgrav_accel.F90:299-314), then the other sinks directly.  One block
+// per sink walks breadth first, a thread per cell of a level (one thread alone
+// took 0.35 ms a sink on a 50000-particle disc); its sums are added in a fixed order.
+constexpr int SW_T = 256;
+__global__ void __launch_bounds__(SW_T) k_sink_walk(
+    int s0, int nsink, const double* __restrict__ sinks, const double4* __restrict__ pm,
+    const double2* __restrict__ hz, GravTree t, const double4* __restrict__ tabG,
+    int* __restrict__ scratch, int cap, double* __restrict__ out, DevError* err) {
+  __shared__ int wsum[SW_T / 32];
+  __shared__ double red[SW_T / 32][4];
+  const int s = s0 + blockIdx.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const double* sr = sinks + s * 5;
   const double rx = sr[0], ry = sr[1], rz = sr[2];
   const double invhp = 1.0 / sr[4];
   const double hp = 1.0 / invhp;
   double cx = 0.0, cy = 0.0, cz = 0.0, cp = 0.0, px = 0.0, py = 0.0, pz = 0.0, pp = 0.0;
-  int c = 0, visits = 0;
-  const int cap = t.ctot + 2;
-  while (true) {
-    if (++visits > cap) {
-      set_error(err, SEREN_GPU_ERR_WALK, KID_SINK, s, c);
+  int* fa = scratch + (size_t)blockIdx.x * 2 * cap;
+  int* fb = fa + cap;
+  if (threadIdx.x == 0) fa[0] = 0;
+  __syncthreads();
+  int nf = 1;
+  while (nf > 0) {
+    int nnext = 0;
+    for (int base = 0; base < nf; base += SW_T) {
+      int nk = 0, kid = 0;
+      if (base + threadIdx.x < nf) {
+        const int c = fa[base + threadIdx.x];
+        const int4 lk = t.link[c];
+        bool open = lk.x == 1;                       // a one-particle leaf has no MAC test
+        if (!open) {
+          const double4 a = t.gA[c];
+          const double d0 = rx - a.x, d1 = ry - a.y, d2 = rz - a.z;
+          const double2 cc = t.gC[c];
+          open = !((d0 * d0 + d1 * d1) + d2 * d2 > cc.y);
+          if (!open) {
+            const double4 q = t.gB[c];
+            cell_term64(d0, d1, d2, a.w, q, make_double2(cc.x, -(q.x + q.z)), cx, cy, cz, cp);
+          }
+        }
+        if (open) {
+          for (int k = 0; k < lk.x; ++k) {
+            const double4 Q = pm[lk.w + k];
+            meanh_term64(Q.x - rx, Q.y - ry, Q.z - rz, 0.5 * (hp + hz[lk.w + k].x), Q.w, tabG, px,
+                         py, pz, pp);
+          }
+          if (lk.x == 0) {
+            nk = t.nkids[c];
+            kid = lk.z;
+          }
+        }
+      }
+      const int inc = warp_incl(nk, lane);
+      if (lane == 31) wsum[w] = inc;
+      __syncthreads();
+      int o = nnext + inc - nk, tot = 0;
+      for (int ww = 0; ww < SW_T / 32; ++ww) {
+        if (ww < w) o += wsum[ww];
+        tot += wsum[ww];
+      }
+      for (int k = 0; k < nk; ++k)
+        if (o + k < cap) fb[o + k] = kid + k;
+      nnext += tot;
+      __syncthreads();
+    }
+    if (nnext > cap) {                               // (a level has at most ctot + 1 cells)
+      if (threadIdx.x == 0) set_error(err, SEREN_GPU_ERR_WALK, KID_SINK, s, nnext);
       break;
     }
-    const int4 lk = t.link[c];
-    if (lk.x == 1) {
-      const double4 Q = pm[lk.w];
-      meanh_term64(Q.x - rx, Q.y - ry, Q.z - rz, 0.5 * (hp + hz[lk.w].x), Q.w, tabG, px, py, pz, pp);
-      c = lk.y;
-    } else {
-      const double4 a = t.gA[c];
-      const double d0 = rx - a.x, d1 = ry - a.y, d2 = rz - a.z;
-      const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
-      const double2 cc = t.gC[c];
-      if (drsqd > cc.y) {
-        const double4 q = t.gB[c];
-        cell_term64(d0, d1, d2, a.w, q, make_double2(cc.x, -(q.x + q.z)), cx, cy, cz, cp);
-        c = lk.y;
-      } else if (lk.x > 0) {
-        for (int k = 0; k < lk.x; ++k) {
-          const double4 Q = pm[lk.w + k];
-          meanh_term64(Q.x - rx, Q.y - ry, Q.z - rz, 0.5 * (hp + hz[lk.w + k].x), Q.w, tabG, px, py,
-                       pz, pp);
-        }
-        c = lk.y;
-      } else if (lk.x == 0) {
-        c = lk.z;
-      } else {
-        c = lk.y;
-      }
-    }
-    if (c > t.ctot) break;
+    int* tmp = fa;
+    fa = fb;
+    fb = tmp;
+    nf = nnext;
   }
-  double ax = cx + px, ay = cy + py, az = cz + pz, pot = cp + pp;
+  double v[4] = {cx + px, cy + py, cz + pz, cp + pp};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(FULLMASK, v[k], o);
+    if (lane == 0) red[w][k] = v[k];
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double ax = 0.0, ay = 0.0, az = 0.0, pot = 0.0;
+  for (int ww = 0; ww < SW_T / 32; ++ww) {
+    ax += red[ww][0];
+    ay += red[ww][1];
+    az += red[ww][2];
+    pot += red[ww][3];
+  }
   double sx = 0.0, sy = 0.0, sz = 0.0, sp = 0.0;
   for (int ss = 0; ss < nsink; ++ss) {
     if (ss == s) continue;
@@ -1022,7 +1063,7 @@ __global__ void k_sink_walk(int nsink, const double* __restrict__ sinks, const d
 
 inline int nb(long n, int t) { return (int)((n + t - 1) / t); }
 
-GravTree grav_tree(const Ctx& c) { return GravTree{c.link, c.gA, c.gB, c.gC, c.info.ctot}; }
+GravTree grav_tree(const Ctx& c) { return GravTree{c.link, c.gA, c.gB, c.gC, c.nkids, c.info.ctot}; }
 
 }  // namespace
 
@@ -1119,8 +1160,17 @@ void launch_grav(Ctx& c, int nact, int nsink, const double* d_sinks, double* ama
 
 void launch_sink_walk(Ctx& c, int nsink, const double* d_sinks, double* d_out) {
   if (nsink <= 0) return;
-  k_sink_walk<<<nb(nsink, 32), 32, 0, c.st>>>(nsink, d_sinks, c.pm, c.hz, grav_tree(c), c.tabG,
-                                              d_out, c.d_err); ++c.nlaunch;
+  // two frontiers per sink in the walk stacks; the sinks in as many rounds as
+  // frontiers of a whole level each allow
+  const long room = 2l * c.wstack_slots * c.wstack_cap;
+  const int cap = (int)std::min<long>(room / 2, c.info.ctot + 1);
+  const int per = (int)std::min<long>(nsink, std::max(1l, room / (2l * cap)));
+  for (int s0 = 0; s0 < nsink; s0 += per) {
+    k_sink_walk<<<std::min(per, nsink - s0), SW_T, 0, c.st>>>(
+        s0, nsink, d_sinks, c.pm, c.hz, grav_tree(c), c.tabG, reinterpret_cast<int*>(c.wstack), cap,
+        d_out, c.d_err);
+    ++c.nlaunch;
+  }
 }
 
 }  // namespace seren
