@@ -452,15 +452,12 @@ __device__ __forceinline__ int gr_next(int* work, int lane) {
 // k_gradh_wide (one block per particle, walks split over subtrees).
 constexpr int GH_LEAVES = 256;   // candidates (or, for the neighbour walk, leaves) per particle
 constexpr int GH_B = 64;         // particles of opened leaves tested at a time
-constexpr int GH_LS = GH_B + 4;  // list stride: an odd number of words
 
 // k_gradh_walk's per-warp shared state beside the walk's
 struct GhShared {
   GrShared w;
   float x[GH_B], y[GH_B], z[GH_B];   // a batch: positions relative to the group's first particle
   int id[GH_B];
-  unsigned char pick[32 * GH_LS];    // each particle's candidates of the batch
-  int cnt[32], tot[32], p[32];
 };
 
 // groups, lpw: as k_grav_walk (a group of 2^lpw particles per warp)
@@ -530,10 +527,8 @@ __global__ void __launch_bounds__(GR_THREADS) k_gradh_walk(
       const float Rm = fmaf(2.0e-6f, um + R32, R32) * 1.000002f;
       const float T = live ? Rm * Rm * 1.000002f : -1.0f;
       const f2 nx = pk1(-ux), ny = pk1(-uy), nz = pk1(-uz), nT = pk1(-T);
-      if (lane < PW) {
-        H.tot[lane] = 0;
-        H.p[lane] = p;
-      }
+      int* const out = rows + (size_t)p * GH_LEAVES;
+      n = 0;
       // the opened leaves' particles, in batches
       int nb = 0, l0 = 0, done = 0;
       while (l0 < nent) {
@@ -575,8 +570,6 @@ __global__ void __launch_bounds__(GR_THREADS) k_gradh_walk(
           H.z[e] = z;
         }
         __syncwarp();
-        int np = 0;
-        unsigned char* row = H.pick + (lane & (PW - 1)) * GH_LS;
 #pragma unroll 1
         for (int c = 0; c < nb; c += 32) {
           unsigned wd = 0u;
@@ -600,27 +593,14 @@ __global__ void __launch_bounds__(GR_THREADS) k_gradh_walk(
           if (lane < PW) {
             while (wd != 0u) {
               const int b = __clz(wd);
-              row[np++] = (unsigned char)(c + b);
+              if (n < GH_LEAVES) out[n] = H.id[c + b];
+              ++n;
               wd ^= 0x80000000u >> b;
             }
           }
         }
-        if (lane < PW) H.cnt[lane] = np;
-        __syncwarp();
-        // to the rows, eight lanes per particle
-        for (int j0 = 0; j0 < PW; j0 += 4) {
-          const int j = j0 + (lane >> 3);
-          const int nj = H.cnt[j], tj = H.tot[j];
-          int* out = rows + (size_t)H.p[j] * GH_LEAVES + tj;
-          for (int k = lane & 7; k < nj; k += 8)
-            if (tj + k < GH_LEAVES) out[k] = H.id[H.pick[j * GH_LS + k]];
-        }
-        __syncwarp();
-        if (lane < PW) H.tot[lane] += np;
         nb = 0;
       }
-      __syncwarp();
-      n = lane < PW ? H.tot[lane] : 0;
       if (n > GH_LEAVES) n = -1;
     }
     if (live && lane < PW) {
@@ -978,24 +958,25 @@ __device__ int rd_walk(const HydroTree& t, int root, int lane, int* fa, int* fb,
     for (int base = 0; base < nf; base += 32) {
       const int idx = base + lane;
       const bool valid = idx < nf;
-      const int c = valid ? fa[idx] : 0;
-      const bool pass = valid && test(c);
-      const int4 lk = t.link[c];
-      const bool isleaf = pass && lk.x > 0;
-      const bool isbr = pass && lk.x == 0;
+      const int c = valid ? fa[idx] : root;
+      const float4 na = t.hN[2 * c], nr = t.hN[2 * c + 1];   // the whole node in one sector
+      const int cn = __float_as_int(nr.z), first = __float_as_int(nr.y);
+      const bool pass = valid && test(c, na, nr.x);
+      const bool isleaf = pass && cn > 0;
+      const bool isbr = pass && cn < 0;
       const unsigned ml = __ballot_sync(FULL, isleaf);
       if (isleaf) {
         const int pos = nleaf + __popc(ml & ((1u << lane) - 1u));
-        if (pos < cap) leaves[pos] = lk.w * 8 + (lk.x - 1);
-        mine += lk.x;
+        if (pos < cap) leaves[pos] = first * 8 + (cn - 1);
+        mine += cn;
       }
       nleaf += __popc(ml);
-      const int nk = isbr ? t.nkids[c] : 0;
+      const int nk = isbr ? -cn : 0;
       const int sc = warp_iscan(nk, lane);
       if (isbr) {
         const int o = nnext + sc - nk;
         for (int j = 0; j < nk; ++j)
-          if (o + j < cap) fb[o + j] = lk.z + j;
+          if (o + j < cap) fb[o + j] = first + j;
       }
       nnext += __shfl_sync(FULL, sc, 31);
     }
@@ -1022,7 +1003,16 @@ __device__ int neib_each(int p, const double4& P, double hp, const double4* __re
                          int cap, int* cand, int lane, DevError* err, F&& f) {
   const double hsp = (KERNRANGESQD * hp) * hp;
   const double R = KERNRANGE * hp;
-  auto test = [&](int c) {
+  const TreeFrame fr = frame_for(t, p);
+  const float px = (float)(P.x - fr.rootx), py = (float)(P.y - fr.rooty),
+              pz = (float)(P.z - fr.rootz), R32 = (float)R;
+  auto test = [&](int c, const float4& h32, float hr32) {
+    const float f0 = h32.x - px, f1 = h32.y - py, f2 = h32.z - pz;
+    const float d2s = (f0 * f0 + f1 * f1) + f2 * f2;
+    const int r1 = test32(d2s, R32 + h32.w, fr.delta);
+    const int r2 = test32(d2s, hr32 + h32.w, fr.delta);
+    if (r1 == 1 || r2 == 1) return true;
+    if (r1 == 0 && r2 == 0) return false;
     const double4 h = t.hA[c];
     const double d0 = h.x - P.x, d1 = h.y - P.y, d2 = h.z - P.z;
     const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
@@ -1039,7 +1029,7 @@ __device__ int neib_each(int p, const double4& P, double hp, const double4* __re
     const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
     return drsqd <= hsp || drsqd <= hsq;
   };
-  const int root = frame_for(t, p).root;
+  const int root = fr.root;
   int* fa = scratch;
   int* lv = scratch + 2 * (size_t)cap;
   int cnt = 0, kept = 0;
@@ -1098,8 +1088,7 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
     gh_init(s, hz[p].x, rextent);
     double Rw = 0.0;
     float R32 = 0.0f;
-    auto gather_test = [&](int c) {                    // BHhydrowalk_hgather.F90:36-40
-      const float4 h32 = t.hA32[c];
+    auto gather_test = [&](int c, const float4& h32, float) {   // BHhydrowalk_hgather.F90:36-40
       const float d0 = h32.x - px, d1 = h32.y - py, d2 = h32.z - pz;
       const int r = test32((d0 * d0 + d1 * d1) + d2 * d2, R32 + h32.w, fr.delta);
       if (r >= 0) return r == 1;
@@ -1268,8 +1257,7 @@ __global__ void __launch_bounds__(HG_THREADS) k_hgather(
     double Rw = KERNRANGE * (HMULT * (HMULT * hz[p].x));    // the reference's first search radius
     if (!(Rw > 0.0) || !isfinite(Rw)) Rw = ldexp(rcap, -12);  // the guess does not change h
     float R32 = 0.0f;
-    auto gather_test = [&](int c) {                     // BHhydrowalk_hgather.F90:36-40
-      const float4 h32 = t.hA32[c];
+    auto gather_test = [&](int c, const float4& h32, float) {   // BHhydrowalk_hgather.F90:36-40
       const float d0 = h32.x - px, d1 = h32.y - py, d2 = h32.z - pz;
       const int r = test32((d0 * d0 + d1 * d1) + d2 * d2, R32 + h32.w, fr.delta);
       if (r >= 0) return r == 1;
@@ -2426,11 +2414,19 @@ void launch_gradh(Ctx& c, int nact) {
       ngrp, gl, lpw, c.pm, c.hz, c.vel, c.rho, c.omega, c.div_v, c.drhodt, c.tabA, c.prm.h_fac,
       c.prm.pp_gather, c.info.rextent, c.leaves, c.nleaf, c.npot, c.redo, c.work + 1,
       c.pplist, c.prm.pp_limit, c.d_err, counts, c.work, t.cl, t.ncl, rec ? 1 : 0, c.pptot);
-  // three walk-stack slots of scratch per redo warp
-  k_gradh_redo<<<std::max(1, (c.wstack_slots / 3) / RD_WARPS), RD_THREADS, 0, c.st>>>(
+  // three walk buffers of wstack_cap entries per redo warp (a walk-stack slot holds
+  // two), for as many warps as fit or as there are buffers for
+  static int rocc[16] = {};
+  int& ro = rocc[c.dev >= 0 && c.dev < 16 ? c.dev : 0];
+  if (ro == 0) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ro, k_gradh_redo, RD_THREADS, 0);
+    if (ro < 1) ro = 1;
+  }
+  const int rblocks = std::min(sm_count(c) * ro, (2 * c.wstack_slots / 3) / RD_WARPS);
+  k_gradh_redo<<<std::max(1, rblocks), RD_THREADS, 0, c.st>>>(
       c.redo, c.work + 1, c.pm, c.hz, c.vel, c.rho, c.omega, c.div_v, c.drhodt, t, c.tabA,
       c.prm.h_fac, c.prm.pp_gather, c.info.rextent, reinterpret_cast<int*>(c.wstack),
-      c.prm.redo_cap > 0 ? std::min(c.prm.redo_cap, 2 * c.wstack_cap) : 2 * c.wstack_cap,
+      c.prm.redo_cap > 0 ? std::min(c.prm.redo_cap, c.wstack_cap) : c.wstack_cap,
       c.wide, c.work + 2, c.leaves, c.d_err, counts);
   // the particles whose walks outgrew the redo kernel's scratch: rounds of
   // whole-GPU walks until each has taken its last step
@@ -2954,26 +2950,29 @@ static __device__ __align__(256) double g_noalloc_scratch[NA_TOTAL];
 
 // Copies the caller's rows into the kernel's layout and checks the lists:
 // 0 <= pptot <= pp_limit (rows the context entry point would complete with a
-// tree walk are refused here) and every listed id in 0..n-1.
+// tree walk are refused here) and every listed id in 0..n-1; NA_SUB threads per
+// row (one thread reading a row alone was 20 us of an 84 us call).
+constexpr int NA_SUB = 16;
 __global__ void k_noalloc_pack(int n, const double* __restrict__ parray,
                                const double* __restrict__ v, const int* __restrict__ pptot,
                                const int* __restrict__ pplist, int L, double4* __restrict__ pm,
                                double2* __restrict__ hz, double4* __restrict__ vel,
                                DevError* err) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = gi / NA_SUB, sub = gi % NA_SUB;
   if (i >= n) return;
-  const double* r = parray + (size_t)i * 6;
-  pm[i] = make_double4(r[0], r[1], r[2], r[3]);
-  hz[i] = make_double2(r[4], r[5]);
-  const double* u = v + (size_t)i * 3;
-  vel[i] = make_double4(u[0], u[1], u[2], 0.0);
   const int nn = pptot[i];
-  if (nn < 0 || nn > L) {
-    set_error(err, SEREN_GPU_ERR_CAPACITY, KID_HYDRO, i, nn);
-    return;
+  if (sub == 0) {
+    const double* r = parray + (size_t)i * 6;
+    pm[i] = make_double4(r[0], r[1], r[2], r[3]);
+    hz[i] = make_double2(r[4], r[5]);
+    const double* u = v + (size_t)i * 3;
+    vel[i] = make_double4(u[0], u[1], u[2], 0.0);
+    if (nn < 0 || nn > L) set_error(err, SEREN_GPU_ERR_CAPACITY, KID_HYDRO, i, nn);
   }
+  if (nn < 0 || nn > L) return;
   const int* row = pplist + (size_t)i * L;
-  for (int k = 0; k < nn; ++k) {
+  for (int k = sub; k < nn; k += NA_SUB) {
     const int q = row[k];
     if (q < 0 || q >= n) {
       set_error(err, SEREN_GPU_ERR_ARG, KID_HYDRO, i, q);
@@ -3074,7 +3073,7 @@ extern "C" int seren_gpu_hydro_forces_noalloc(int32_t n, const double* parray, c
   const double4* tab = reinterpret_cast<const double4*>(base + NA_TAB + kernel * NA_TABLEN);
   // the array keeps the previous call's contents: only the error block must start at zero
   if (cudaMemsetAsync(d_err, 0, sizeof(DevError), st) != cudaSuccess) return SEREN_GPU_ERR_CUDA;
-  if (noalloc_launch(k_noalloc_pack, nb(n, 256), 256, st, n, parray, v, pptot, pplist, pp_limit,
+  if (noalloc_launch(k_noalloc_pack, nb((long)n * NA_SUB, 256), 256, st, n, parray, v, pptot, pplist, pp_limit,
                      pm, hz, vel, d_err) != cudaSuccess)
     return SEREN_GPU_ERR_CUDA;
   if ((rc = noalloc_status(st, d_err))) return rc;
