@@ -38,9 +38,18 @@ struct HydroTree {
   float delta;          // bound on the FP32 rounding of a root-relative coordinate
   int root;             // root cell of the walks
   double rextent;       // root box extent (the grad-h bisection's first h_upper)
+  double unit;          // gh_unit(rextent)
   const CloudInfo* cl;  // a forest of ncl trees (NULL: one tree)
   int ncl;
 };
+
+// A power of two that brings lengths of the order of a root box to between 1/2 and 1
+// (1 for a box without extent)
+__host__ __device__ __forceinline__ double gh_unit(double rextent) {
+  if (!(rextent > 0.0)) return 1.0;
+  const int e = -1 - ilogb(rextent);
+  return scalbn(1.0, e < 1000 ? e : 1000);
+}
 
 // The tree particle p walks: its root cell, root box, rounding bound and
 // extent - in a forest those of its cloud, else the one tree's.  (A local
@@ -456,7 +465,8 @@ constexpr int GH_B = 64;         // particles of opened leaves tested at a time
 // k_gradh_walk's per-warp shared state beside the walk's
 struct GhShared {
   GrShared w;
-  float x[GH_B], y[GH_B], z[GH_B];   // a batch: positions relative to the group's first particle
+  // a batch: positions relative to the group's first particle, in units of the root box
+  float x[GH_B], y[GH_B], z[GH_B];
   int id[GH_B];
 };
 
@@ -519,12 +529,17 @@ __global__ void __launch_bounds__(GR_THREADS) k_gradh_walk(
       // this lane's particle relative to the group's first one, and its radius
       // 2 h_high with a margin for the rounding of either offset (2^-24 of a
       // candidate's, itself at most this lane's plus the radius, and of the
-      // difference and the squares)
+      // difference and the squares); in units of the root box, so that the squares
+      // stay within FP32 whatever the unit of length, the radius cut off far beyond
+      // it (an h of any size, where every particle is a candidate)
       const double fx = __shfl_sync(FULL, rx, 0), fy = __shfl_sync(FULL, ry, 0),
                    fz = __shfl_sync(FULL, rz, 0);
-      const float ux = (float)(rx - fx), uy = (float)(ry - fy), uz = (float)(rz - fz);
+      const double unit = t.cl ? gh_unit(fr.rextent) : t.unit;
+      const float ux = (float)((rx - fx) * unit), uy = (float)((ry - fy) * unit),
+                  uz = (float)((rz - fz) * unit);
       const float um = fabsf(ux) + fabsf(uy) + fabsf(uz);
-      const float Rm = fmaf(2.0e-6f, um + R32, R32) * 1.000002f;
+      const float Ru = fminf((float)(Rw * unit), 1.0e15f);
+      const float Rm = fmaf(2.0e-6f, um + Ru, Ru) * 1.000002f;
       const float T = live ? Rm * Rm * 1.000002f : -1.0f;
       const f2 nx = pk1(-ux), ny = pk1(-uy), nz = pk1(-uz), nT = pk1(-T);
       int* const out = rows + (size_t)p * GH_LEAVES;
@@ -558,12 +573,12 @@ __global__ void __launch_bounds__(GR_THREADS) k_gradh_walk(
 #pragma unroll
         for (int u = 0; u < GH_B / 32; ++u) {
           const int e = 32 * u + lane;
-          float x = 3.0e38f, y = 3.0e38f, z = 3.0e38f;
+          float x = 0.0f, y = 0.0f, z = 0.0f;
           if (e < nb) {
             const double4 Q = pm[H.id[e]];
-            x = (float)(Q.x - fx);
-            y = (float)(Q.y - fy);
-            z = (float)(Q.z - fz);
+            x = (float)((Q.x - fx) * unit);
+            y = (float)((Q.y - fy) * unit);
+            z = (float)((Q.z - fz) * unit);
           }
           H.x[e] = x;
           H.y[e] = y;
@@ -590,6 +605,7 @@ __global__ void __launch_bounds__(GR_THREADS) k_gradh_walk(
             wd = __funnelshift_l(__float_as_uint(d2), wd, 1);
             wd = __funnelshift_l(__float_as_uint(d3), wd, 1);
           }
+          if (nb - c < 32) wd &= ~(FULL >> (nb - c));     // only the batch's own slots
           if (lane < PW) {
             while (wd != 0u) {
               const int b = __clz(wd);
@@ -2318,7 +2334,7 @@ HydroTree hydro_tree(const Ctx& c) {
   const double delta = ldexp(1.0, -22) * (c.info.cellsize > 0.0 ? c.info.cellsize : 1.0);
   return HydroTree{c.link, c.hA, c.hrm, c.hA32, c.hrm32, c.nkids, c.hN, c.info.ctot, c.info.root[0],
                    c.info.root[1], c.info.root[2], (float)delta, 0, c.info.rextent,
-                   c.ncloud > 1 ? c.d_clouds : nullptr, c.ncloud};
+                   gh_unit(c.info.rextent), c.ncloud > 1 ? c.d_clouds : nullptr, c.ncloud};
 }
 
 }  // namespace
