@@ -275,6 +275,15 @@ __global__ void k_gather_hi(const unsigned long long* __restrict__ hi, const int
   keys[i] = hi[idx[i]];
 }
 
+// the lo words in the order of the sorted keys (k_cells_emit reorders idx while other
+// blocks still compare keys, so it cannot look them up through idx)
+__global__ void k_gather_lo(const unsigned* __restrict__ lo, const int* __restrict__ idx, int n,
+                            unsigned* __restrict__ sorted) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  sorted[i] = lo[idx[i]];
+}
+
 // ---------------------------------------------------------------------------
 // stable LSD radix sort of (64-bit key, int) pairs, 8-bit digits
 constexpr int RS_T = 256;
@@ -484,13 +493,11 @@ __global__ void __launch_bounds__(SS_T) k_small_sort(unsigned long long* __restr
 // level split took 10 and 2 for each level (60-70 us a level).
 constexpr int CE_T = 256;
 
-// Sorted keys: levels 1..21 in keys, 22..30 in lo (input order, with deep); levels
-// beyond `ordered` are not sorted and count as shared.
+// Sorted keys: levels 1..21 in keys, 22..30 in lo (NULL: none); levels beyond
+// `ordered` are not sorted and count as shared.
 struct SortedKeys {
   const unsigned long long* keys;
   const unsigned* lo;
-  const int* idx;
-  int deep;
   int ordered;
 };
 
@@ -498,7 +505,7 @@ __device__ __forceinline__ int share_levels(unsigned long long a, unsigned long 
                                             unsigned la, unsigned lb, const SortedKeys& k) {
   const unsigned long long x = a ^ b;
   int c = x == 0ull ? KEY_LEVELS : (__clzll(x) - 1) / 3;
-  if (x == 0ull && k.deep) {
+  if (x == 0ull && k.lo) {
     const unsigned y = la ^ lb;
     c += y == 0u ? LO_LEVELS : (__clz(y) - 5) / 3;
   }
@@ -521,7 +528,7 @@ __global__ void __launch_bounds__(CE_T) k_cells_mark(int n, SortedKeys K,
     const int i = base - H + t;
     const bool in = i >= 0 && i < n;
     sk[t] = in ? K.keys[i] : 0ull;
-    sl[t] = in && K.deep ? K.lo[K.idx[i]] : 0u;
+    sl[t] = in && K.lo ? K.lo[i] : 0u;
     sc[t] = !in ? -1 : cl ? cloud_of(cl, ncl, i) : 0;
   }
   __syncthreads();
@@ -626,7 +633,7 @@ __global__ void __launch_bounds__(CE_T) k_cells_emit(
   const int cloud_end = hi;
   const int l0 = __ffs(m) - 1, leaf = 31 - __clz(m);
   const unsigned long long key = K.keys[i];
-  const unsigned lo = K.deep ? K.lo[K.idx[i]] : 0u;
+  const unsigned lo = K.lo ? K.lo[i] : 0u;
   for (int l = l0; l <= leaf; ++l) {
     int end;
     if (l == 0) {
@@ -638,7 +645,7 @@ __global__ void __launch_bounds__(CE_T) k_cells_emit(
       int a = i + LEAFMAX + 1, b = hi;
       while (a < b) {
         const int mid = a + ((b - a) >> 1);
-        if (share_levels(key, K.keys[mid], lo, K.deep ? K.lo[K.idx[mid]] : 0u, K) >= l) a = mid + 1;
+        if (share_levels(key, K.keys[mid], lo, K.lo ? K.lo[mid] : 0u, K) >= l) a = mid + 1;
         else b = mid;
       }
       end = a;
@@ -1134,7 +1141,12 @@ static int build_cells(Ctx& c, bool deep, int ordered) {
   const int n = c.ptot;
   const int ncl = c.ncloud;
   const CloudInfo* cl = ncl > 1 ? c.d_clouds : nullptr;
-  const SortedKeys K{c.keys, c.keys_lo, c.idx, deep ? 1 : 0, ordered};
+  unsigned* lo = nullptr;
+  if (deep) {
+    lo = reinterpret_cast<unsigned*>(c.keys_alt);               // free after the sort
+    k_gather_lo<<<nb(n, 256), 256, 0, c.st>>>(c.keys_lo, c.idx, n, lo); ++c.nlaunch;
+  }
+  const SortedKeys K{c.keys, lo, ordered};
   unsigned* mask = reinterpret_cast<unsigned*>(c.idx_alt);      // free after the sort
   const int nblk = nb(n, CE_T);
   k_cells_mark<<<nblk, CE_T, 0, c.st>>>(n, K, cl, ncl, mask, c.blk_count, nblk);

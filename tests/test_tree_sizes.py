@@ -5,7 +5,7 @@ particles; cells and order bit for bit against the oracle."""
 import numpy as np
 import pytest
 
-from helpers import params
+from helpers import deep_clump, params
 from oracle.oracle import Oracle
 from seren_b200 import ics
 
@@ -49,5 +49,17 @@ def test_shallow_tree_after_a_deep_one_and_back():
     g, o = GpuHotPath(n, params(flat)), Oracle(n, params(flat))
     depths = [_compare(g, o, ic["parray"]) for ic in (flat, deep, deep, flat, flat, deep)]
     assert max(depths[1:3]) > 10 and depths[0] <= 10 and depths[3] <= 10
+    g.close()
+    o.close()
+
+
+def test_deep_tree_of_many_blocks():
+    """24 levels and 80000 particles: the cells are written while other blocks put
+    their leaves' particles into input order."""
+    from seren_b200.gpu import GpuHotPath
+    ic = deep_clump(1.0e-5, n_core=40000, n_halo=40000)
+    n = ic["parray"].shape[0]
+    g, o = GpuHotPath(n, params(ic)), Oracle(n, params(ic))
+    assert _compare(g, o, ic["parray"]) > 21
     g.close()
     o.close()
