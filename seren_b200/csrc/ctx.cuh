@@ -169,9 +169,10 @@ struct Ctx {
   bool sink_a_valid = false;
   std::vector<double> sink_rmh, sink_v, sink_a, sink_pot, sink_radius, sink_rold, sink_vold,
       sink_vhalf;
-  int* leaves = nullptr;      // [pmax][256] opened leaves of each particle's grad-h walk
-  int* nleaf = nullptr;       // their number (-1: overflow)
-  int* npot = nullptr;        // [pmax] particles in those leaves (pp_pot)
+  int* leaves = nullptr;      // [pmax][256] a walk's candidates or opened leaves per particle (sph.cu)
+  int* nleaf = nullptr;       // their number (negative: leaves, or overflow)
+  int* npot = nullptr;        // [pmax] particles in the opened leaves (pp_pot); after grad-h the
+                              // gather neighbours recorded (-1: none)
   int* redo = nullptr;        // [pmax] particles whose grad-h is redone alone; count in work[1]
   int* wide = nullptr;        // [pmax] particles whose grad-h walks cover most of the tree; count in work[2]
   void* wst = nullptr;        // state of a batch of those particles (sph.cu)

@@ -446,20 +446,28 @@ __device__ __forceinline__ int gr_next(int* work, int lane) {
 // (:154-170, BHhydrowalk_hgather at h_high = h*HMULT), one group walk per warp;
 // the particles of the opened leaves are then tested against every particle of
 // the group at once, and each particle's candidates within 2 h_high (a superset,
-// FP32 with a margin) go to its own row of c.leaves (GH_LEAVES ids, in leaf
-// order), their number to c.nleaf (-1 when the row or the walk overflows), the
-// number of particles in the leaves it opened (pp_pot) to c.npot.
+// FP32 with a margin) go to its own row of c.leaves (GH_LEAVES ids, in the order
+// of the walk), their number to c.nleaf, the number of particles in the leaves it
+// opened (pp_pot) to c.npot.  A particle with more candidates than a row holds gets
+// its opened leaves in the row instead (c.nleaf = -1 - their number), and -1 when
+// those do not fit either or the walk overflows.
 //
 // k_gradh_pass: each lane holds one particle's state; the reference's iteration
 // (:154-285) and final pass (:317-425) run over the recorded candidates, which
 // hold every particle within 2h while h <= h_high.  The reference leaves this
 // path only to grow h (pp_pot < pp_gather) or to walk again (h > h_high); a
-// particle that needs either, whose final h reaches h_high, or whose row
-// overflowed, is redone from the start with walks of its own, which take the
-// reference's steps in the same order: k_gradh_redo (one warp per particle, walk
-// buffers in global scratch) and, for walks too large for those buffers,
-// k_gradh_wide (one block per particle, walks split over subtrees).
-constexpr int GH_LEAVES = 256;   // candidates (or, for the neighbour walk, leaves) per particle
+// particle that needs either, whose final h reaches h_high, or whose row holds
+// no candidates, goes to k_gradh_redo (one warp per particle), which runs the
+// reference's steps in the same order over the opened leaves, those of its row or
+// of walks of its own (buffers in global scratch), and, for walks too large for
+// those buffers, to the whole-GPU rounds (k_wide_*).
+//
+// Row capacity: about 33.5 (1.1 h_fac)^3 candidates, 77 at h_fac = 1.2; above 256
+// from h_fac = 1.8 on, or where the h that comes in is 1.5 times the right one
+// (the guess of a first call).  1M core at h_fac = 2: grad-h 21.7 ms and the
+// neighbour lists 1.2; 24.9 and 403 when a particle whose row overflowed was walked
+// again for its h and once more for its neighbours.
+constexpr int GH_LEAVES = 256;   // candidates or leaves of a row
 constexpr int GH_B = 64;         // particles of opened leaves tested at a time
 
 // k_gradh_walk's per-warp shared state beside the walk's
@@ -617,7 +625,18 @@ __global__ void __launch_bounds__(GR_THREADS) k_gradh_walk(
         }
         nb = 0;
       }
-      if (n > GH_LEAVES) n = -1;
+      // a row that overflows: the lane's opened leaves
+      const bool big = live && lane < PW && n > GH_LEAVES;
+      if (__any_sync(FULL, big)) {
+        int k = 0;
+        for (int e = 0; e < nent; ++e) {
+          if (big && ((R.mask[e] >> lane) & 1u)) {
+            if (k < GH_LEAVES) out[k] = R.code[e];
+            ++k;
+          }
+        }
+        if (big) n = k <= GH_LEAVES ? -1 - k : -1;
+      }
     }
     if (live && lane < PW) {
       nrow[p] = n;
@@ -939,7 +958,6 @@ __global__ void __launch_bounds__(GP_THREADS, 8) k_gradh_pass(
     if (single) {
       ++nsingle;
       redo[atomicAdd(nredo, 1)] = p;
-      if (rec) npot[p] = -1;                       // its neighbour list: from a walk
     }
   }
   warp_count(counts + 5, npass, lane);
@@ -950,11 +968,13 @@ __global__ void __launch_bounds__(GP_THREADS, 8) k_gradh_pass(
 
 // ---------------------------------------------------------------------------
 // grad-h for the particles k_gradh_pass hands back (redo[0..*nredo)): one warp
-// per particle runs the reference's loop (:132-425) with walks of its own.  A
-// walk runs breadth-first with the lanes spread over the cells of a level; its
-// two frontiers and the opened leaves live in global scratch (three walk-stack
-// slots per warp, idle while this kernel runs), and the passes flatten the
-// leaves GP_SEG at a time and share the candidates out over the lanes.
+// per particle runs the reference's loop (:132-425), from the leaves of its row
+// where the group walk left them there, else with walks of its own.  A walk runs
+// breadth-first with the lanes spread over the cells of a level; its two frontiers
+// and the opened leaves live in global scratch (three buffers of cap entries per
+// warp in the walk stacks, idle while this kernel runs), and the passes flatten
+// the leaves GP_SEG at a time and share the candidates out over the lanes.  The
+// final pass records the gather neighbours (rec) as k_gradh_pass does.
 constexpr int RD_THREADS = 128;
 constexpr int RD_WARPS = RD_THREADS / 32;
 
@@ -1082,7 +1102,9 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
     double* __restrict__ omega, double* __restrict__ divv, double* __restrict__ drhodt,
     HydroTree t, const double4* __restrict__ tabA, double h_fac, int pp_gather, double rextent0,
     int* __restrict__ scratch, int cap, int* __restrict__ wide, int* __restrict__ nwide,
-    int* __restrict__ leaves, DevError* err, unsigned long long* counts) {
+    int* __restrict__ leaves, const int* __restrict__ nrow, int* __restrict__ npot,
+    int* __restrict__ gset, int L, int rec, int* __restrict__ pptot, DevError* err,
+    unsigned long long* counts) {
   __shared__ int cand_all[RD_WARPS][GP_SEG * LEAFMAX];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int* cand = cand_all[w];
@@ -1114,6 +1136,13 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
       return ((e0 * e0 + e1 * e1) + e2 * e2) <= tt * tt;
     };
     int nl = 0;
+    const int* lf = lv;
+    if (const int row = nrow[p]; row < -1) {           // walked at h*HMULT (:154-170)
+      lf = leaves + (size_t)p * GH_LEAVES;
+      nl = -1 - row;
+      s.h_high = s.hp * HMULT;
+      s.pp_pot = npot[p];
+    }
     bool over = false, bad = false;
     while (true) {
       while (true) {                                                   // :154-191
@@ -1125,6 +1154,7 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
           ++nwalk;
           nl = rd_walk(t, fr.root, lane, fa, fb, lv, cap, cnt, nvisit, gather_test);
           if (nl < 0) { over = true; break; }
+          lf = lv;
           s.pp_pot = cnt;
         }
         if (s.pp_pot < pp_gather) {
@@ -1141,7 +1171,7 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
       const double hs = (KERNRANGESQD * s.hp) * s.hp;
       double part = 0.0;
       for (int s0 = 0; s0 < nl; s0 += GP_SEG) {
-        const int nc = gp_flatten(lv + s0, min(GP_SEG, nl - s0), cand, lane);
+        const int nc = gp_flatten(lf + s0, min(GP_SEG, nl - s0), cand, lane);
         for (int k = lane; k < nc; k += 32) {
           const int q = cand[k];
           const double4 Q = pm[q];
@@ -1154,13 +1184,14 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
       ncands += s.pp_pot;
       if (gh_after_pass(s, mp, h_fac, rextent, (mp * t0.x) * hf + warp_sum(part))) break;
     }
+    if ((over || bad) && rec && lane == 0) npot[p] = -1;   // its neighbour list: from a walk
     if (bad) {
       if (lane == 0) set_error(err, SEREN_GPU_ERR_WALK, KID_GRADH, p, -1);
       continue;
     }
     if (over) {                                        // more than cap leaves or cells a level
       // the whole-GPU path takes the particle from here: its state goes to
-      // its leaf row (no longer read once the particle is redone), and its
+      // its row (no longer read once the particle has walked again), and its
       // next step is the counting walk at s.h_high that outgrew the scratch
       if (lane == 0) {
         *reinterpret_cast<GhState*>(leaves + (size_t)p * GH_LEAVES) = s;
@@ -1175,18 +1206,30 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
     const double4 vp = vel[p];
     GhFinal f;
     f.rt = 0.0; f.om = 0.0; f.dv = 0.0; f.zt = 0.0;
+    // the leaves hold every particle within 2 h_high, so the gather neighbours are
+    // complete while h < h_high
+    const bool record = rec && hp < s.h_high;
+    int gcnt = 0;
     for (int s0 = 0; s0 < nl; s0 += GP_SEG) {
-      const int nc = gp_flatten(lv + s0, min(GP_SEG, nl - s0), cand, lane);
-      for (int k = lane; k < nc; k += 32) {
-        const int q = cand[k];
+      const int nc = gp_flatten(lf + s0, min(GP_SEG, nl - s0), cand, lane);
+      for (int b = 0; b < nc; b += 32) {
+        const int q = b + lane < nc ? cand[b + lane] : p;
         const double4 Q = pm[q];
         const double d0 = Q.x - rx, d1 = Q.y - ry, d2 = Q.z - rz;
         const double drsqd = (d0 * d0 + d1 * d1) + d2 * d2;
-        if (q == p || drsqd > hs) continue;
+        const bool in = q != p && drsqd <= hs;
+        if (record) {
+          const unsigned m = __ballot_sync(FULL, in);
+          const int o = gcnt + __popc(m & ((1u << lane) - 1u));
+          if (in && o < L) gset[(size_t)p * L + o] = q;
+          gcnt += __popc(m);
+        }
+        if (!in) continue;
         const double4 V = vel[q];
         const double dv0 = V.x - vp.x, dv1 = V.y - vp.y, dv2 = V.z - vp.z;
         gh_final_in(drsqd, Q.w, (dv0 * d0 + dv1 * d1) + dv2 * d2, ih, hf, f);
       }
+      __syncwarp();
     }
     ++npass;
     ncands += s.pp_pot;
@@ -1196,7 +1239,11 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
     g.om = g.om + warp_sum(f.om);
     g.dv = g.dv + warp_sum(f.dv);
     g.zt = g.zt + warp_sum(f.zt);
-    if (lane == 0) gh_store(p, mp, hp, g, hz, rho, omega, divv, drhodt, err);
+    if (lane == 0) {
+      gh_store(p, mp, hp, g, hz, rho, omega, divv, drhodt, err);
+      if (rec) npot[p] = record ? gcnt : -1;           // -1: its neighbour list from a walk
+      if (record) pptot[p] = gcnt;
+    }
   }
   if (lane == 0) {
     atomicAdd(counts + 3, nwalk);
@@ -2443,7 +2490,8 @@ void launch_gradh(Ctx& c, int nact) {
       c.redo, c.work + 1, c.pm, c.hz, c.vel, c.rho, c.omega, c.div_v, c.drhodt, t, c.tabA,
       c.prm.h_fac, c.prm.pp_gather, c.info.rextent, reinterpret_cast<int*>(c.wstack),
       c.prm.redo_cap > 0 ? std::min(c.prm.redo_cap, c.wstack_cap) : c.wstack_cap,
-      c.wide, c.work + 2, c.leaves, c.d_err, counts);
+      c.wide, c.work + 2, c.leaves, c.nleaf, c.npot, c.pplist, c.prm.pp_limit, rec ? 1 : 0,
+      c.pptot, c.d_err, counts);
   // the particles whose walks outgrew the redo kernel's scratch: rounds of
   // whole-GPU walks until each has taken its last step
   int nwide = 0;
@@ -2568,8 +2616,8 @@ void launch_neib(Ctx& c, int nact, bool sorted) {
 //  * the grad-h final pass has already applied the test r^2 <= 4h_p^2 with
 //    the final h to candidates that hold every particle within 2h (h <
 //    h_high) and written the gather set to p's row, its size to pptot and npot;
-//    the particles it did not finish (npot = -1), listed in order, get their
-//    whole rows from a walk of their own (k_neib_walked);
+//    the others (npot = -1) are listed and get their whole rows from a walk of
+//    their own (the first blocks of k_neib_transpose);
 //  * k_neib_transpose adds p to the row of each q in p's gather set that does
 //    not have p in its own (r^2 > 4h_q^2): the scatter neighbours;
 //  * k_neib_sort puts each such row in increasing order when the caller reads

@@ -47,3 +47,43 @@ def test_smoothing_lengths_beyond_the_cloud(n, h):
     ic = ics.uniform_sphere(n=n, seed=72)
     ic["parray"][:, 4] = h
     _compare(ic, False)
+
+
+@pytest.mark.parametrize("h_fac", [1.75, 1.85, 2.2])
+def test_rows_that_overflow(h_fac):
+    """About 240, 280 and 480 candidates per particle: rows of 256 that mostly hold
+    them, mostly hold leaves, and hold leaves only."""
+    ic = ics.uniform_sphere(n=20011, seed=73, h_fac=h_fac)
+    ic["v"] = np.random.Generator(np.random.PCG64(74)).normal(0.0, 0.1, ic["v"].shape)
+    _compare(ic, True)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_rows_that_overflow_are_not_walked_again(precision):
+    """In a steady state of more candidates than a row holds a particle's leaves are
+    walked once; the evaluation repeats bit for bit, and its FP64 form agrees with
+    the oracle."""
+    from seren_b200.gpu import GpuHotPath
+    ic = ics.uniform_sphere(n=20011, seed=75, h_fac=2.0)
+    n = ic["parray"].shape[0]
+    out = []
+    for _ in range(2):
+        g = GpuHotPath(n, params(ic, precision=precision))
+        g.upload(ic["parray"], ic["v"], ic["sound"] ** 2)
+        g.force_step(first_call=True)
+        g.force_step()
+        counts = g.last_step_stats()[2]
+        out.append(g.download())
+        g.close()
+        assert counts[15] > n // 2                       # most rows overflow
+        assert counts[3] < 1.1 * n                       # grad-h walks
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
+    if precision == 0:
+        o = Oracle(n, params(ic))
+        p, perm = o.tree_update(ic["parray"])
+        s = o.sph_update(p, ic["v"][perm], first_call=True)
+        p2, perm2 = o.tree_update(s["parray"])
+        s2 = o.sph_update(p2, ic["v"][perm][perm2])
+        o.close()
+        assert rel_rows(out[0]["rho"], s2["rho"]).max() < 1e-10
