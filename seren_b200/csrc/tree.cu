@@ -1336,9 +1336,10 @@ int restock(Ctx& c, bool& rebuilt) {
   return SEREN_GPU_OK;
 }
 
-// the levels 0 .. top-1 with at most TOP_CELLS cells each (level 0 always)
+// the levels 0 .. top-1 with at most TOP_CELLS cells each (none where a forest has
+// more roots: 16000 clouds, tree stage 1.68 ms with the roots in one block, 0.84 without)
 static int top_levels(const Ctx& c) {
-  int top = 1;
+  int top = 0;
   while (top <= c.info.ltot && c.info.last_cell[top] - c.info.first_cell[top] < TOP_CELLS) ++top;
   return top;
 }
@@ -1346,7 +1347,7 @@ static int top_levels(const Ctx& c) {
 static LevelFirst level_first(const Ctx& c, int top) {
   LevelFirst F{};
   for (int l = 0; l < top; ++l) F.first[l] = c.info.first_cell[l];
-  F.first[top] = c.info.last_cell[top - 1] + 1;
+  if (top > 0) F.first[top] = c.info.last_cell[top - 1] + 1;
   return F;
 }
 
@@ -1364,6 +1365,7 @@ void launch_stock(Ctx& c) {
     const int f = c.info.first_cell[l], la = c.info.last_cell[l];
     k_stock_level<<<nb(la - f + 1, 128), 128, 0, c.st>>>(f, la, a); ++c.nlaunch;
   }
+  if (top == 0) return;
   k_stock_top<<<1, TOP_T, 0, c.st>>>(top, level_first(c, top), a); ++c.nlaunch;
 }
 
@@ -1374,6 +1376,7 @@ void launch_update_hmax(Ctx& c) {
     k_hmax_level<<<nb(la - f + 1, 128), 128, 0, c.st>>>(f, la, c.link, c.nkids, c.hz, c.hrm,
                                                         c.hrm32, c.hN); ++c.nlaunch;
   }
+  if (top == 0) return;
   k_hmax_top<<<1, TOP_T, 0, c.st>>>(top, level_first(c, top), c.link, c.nkids, c.hz, c.hrm,
                                     c.hrm32, c.hN); ++c.nlaunch;
 }

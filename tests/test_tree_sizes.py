@@ -63,3 +63,28 @@ def test_deep_tree_of_many_blocks():
     assert _compare(g, o, ic["parray"]) > 21
     g.close()
     o.close()
+
+
+def test_forest_of_more_roots_than_a_block_takes():
+    """1030 clouds: the level of the roots is stocked like any other; some of the
+    clouds against the same clouds alone, bit for bit."""
+    from seren_b200.gpu import GpuHotPath
+    m, ncl = 70, 1030
+    kinds = [ics.uniform_sphere(n=m, seed=80 + k) for k in range(5)]
+    clouds = [kinds[k % 5] for k in range(ncl)]
+    g = GpuHotPath(m * ncl, params(kinds[0]))
+    g.upload(np.vstack([c["parray"] for c in clouds]), np.vstack([c["v"] for c in clouds]),
+             np.concatenate([c["sound"] ** 2 for c in clouds]))
+    g.set_clouds([m] * ncl)
+    g.force_step(first_call=True)
+    st = g.download()
+    g.close()
+    for k, ic in enumerate(kinds):
+        one = GpuHotPath(m, params(ic))
+        one.upload(ic["parray"], ic["v"], ic["sound"] ** 2)
+        one.force_step(first_call=True)
+        s1 = one.download()
+        one.close()
+        for c in (k, ncl - 5 + k):
+            for name in ("parray", "rho", "omega", "a", "gpot"):
+                assert np.array_equal(st[name][c * m:(c + 1) * m], s1[name]), (c, name)
