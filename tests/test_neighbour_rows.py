@@ -48,3 +48,27 @@ def test_sink_forces_of_many_sinks(n, nsink):
     o.close()
     # FP64 sums of up to n terms in another order
     assert rel_rows(ag, ao).max() < 1e-11 and rel_rows(pg, po).max() < 1e-12
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_hydro_after_a_restock(precision):
+    """Rows over pp_limit are searched on the fly, by the cells' search ranges of the
+    last sph_update: a restock of the same particles leaves those as they are.
+    (Smoothing lengths that differ from cell to cell: many neighbours are found by
+    the scatter test only.)"""
+    from seren_b200.gpu import GpuHotPath
+    n = 4001
+    ic = ics.plummer(n=n, seed=64)
+    prm = params(ic, precision=precision)
+    prm.pp_limit = 30
+    g = GpuHotPath(n, prm)
+    p, perm = g.tree_update(ic["parray"])
+    s = g.sph_update(p, ic["v"][perm], first_call=True)
+    assert (s["pptot"] > prm.pp_limit).mean() > 0.5
+    sound = np.full(n, 0.1)
+    press = sound * sound * s["rho"]
+    a = g.hydro_forces(press, sound)
+    g.tree_update(s["parray"], do_build=False)
+    again = g.hydro_forces(press, sound)
+    g.close()
+    assert np.array_equal(a, again)
