@@ -260,7 +260,7 @@ void free_all(Ctx& c) {
                 c.pf, c.hf4,
                 c.pptot, c.pplist, c.stage, c.istage, c.keys, c.keys_alt, c.keys_hi, c.keys_lo, c.idx, c.idx_alt,
                 c.rs_hist, c.bbox_part, c.blk_count, c.bflag, c.bscan, c.pcount, c.parent,
-                c.level, c.nkids, c.work, c.sinks, c.wstack, c.leaves, c.nleaf, c.npot, c.redo, c.wide, c.wst, c.wacc, c.link, c.gA, c.gB, c.gC, c.wA, c.hN, c.hA, c.hrm, c.hA32, c.hrm32, c.hmax, c.bbmin, c.bbmax, c.d_info,
+                c.level, c.nkids, c.work, c.sinks, c.wstack, c.leaves, c.nleaf, c.npot, c.redo, c.wide, c.wst, c.wacc, c.link, c.gA, c.gB, c.gC, c.wA, c.hN, c.hA, c.hrm, c.hmax, c.bbmin, c.bbmax, c.d_info,
                 c.d_err, c.d_counts, c.sink_out, c.tabA, c.tabG, c.scan.total, c.scan.level_buf[0],
                 c.scan.level_buf[1], c.scan.level_buf[2], c.scan.level_buf[3]};
   for (void* p : ps)
@@ -306,7 +306,7 @@ int alloc_all(Ctx& c) {
          alloc(c.rs_hist, rsh) | alloc(c.bbox_part, 6 * 1184) |
          alloc(c.blk_count, 32 * ((P + 255) / 256)) | alloc(c.bflag, C) | alloc(c.bscan, C);
   bad |= alloc(c.pcount, C) | alloc(c.parent, C) | alloc(c.level, C) | alloc(c.link, C);
-  bad |= alloc(c.hA32, C) | alloc(c.hrm32, C) | alloc(c.nkids, C) | alloc(c.work, 4);
+  bad |= alloc(c.nkids, C) | alloc(c.work, 4);
   bad |= alloc(c.leaves, P * 256) | alloc(c.nleaf, P) | alloc(c.npot, P) | alloc(c.redo, P) | alloc(c.wide, P);
   bad |= wide_scratch_alloc(c);
   bad |= alloc(c.gA, C) | alloc(c.gB, C) | alloc(c.gC, C) | alloc(c.wA, 2 * C) | alloc(c.hN, 2 * C) |
@@ -324,7 +324,6 @@ int alloc_all(Ctx& c) {
   cudaMemset(c.d_err, 0, sizeof(DevError));
   cudaMemset(c.d_counts, 0, sizeof(int) * 32);
   cudaMemset(c.hrm, 0, sizeof(double) * C);
-  cudaMemset(c.hrm32, 0, sizeof(float) * C);
   for (auto& e : c.ev)
     if (cudaEventCreate(&e) != cudaSuccess) return -1;
   // kernel tables

@@ -143,14 +143,13 @@ struct Ctx {
   // bits) the first particle of a leaf or first child of a branch, and the
   // leaf's particle count or minus the branch's number of children
   float4* wA = nullptr;
-  // hydro walk node, two float4 per cell: hA32; hrm32, then (as int bits)
+  // hydro walk node, two float4 per cell: FP32 bbox centre - root centre, rmax
+  // rounded up; hrangemax rounded up, then (as int bits)
   // the first particle of a leaf or first child of a branch, and the leaf's
   // particle count or minus the branch's number of children
   float4* hN = nullptr;
   double4* hA = nullptr;      // hydro: bbox centre x, y, z, rmax
   double* hrm = nullptr;      // hydro: hrangemax
-  float4* hA32 = nullptr;     // hydro walk: FP32 centre - root centre, rmax rounded up
-  float* hrm32 = nullptr;     // hydro walk: hrangemax rounded up
   double* hmax = nullptr;     // stock: max h in the cell (at stock time)
   double4* bbmin = nullptr;
   double4* bbmax = nullptr;

@@ -28,10 +28,9 @@ struct HydroTree {
   const int4* link;     // {leaf, nextcell, ifopen, pstart}
   const double4* hA;    // bbox centre, rmax
   const double* hrm;    // hrangemax
-  const float4* hA32;   // FP32 centre - root centre, rmax rounded up
-  const float* hrm32;   // hrangemax rounded up
   const int* nkids;     // children per cell (ids ifopen .. ifopen + nkids - 1)
-  const float4* hN;     // two per cell: hA32; hrm32, first particle / first child,
+  const float4* hN;     // two per cell: FP32 bbox centre - root centre, rmax rounded up;
+                        // hrangemax rounded up, first particle / first child,
                         // leaf count / -children (int bits)
   int ctot;
   double rootx, rooty, rootz;
@@ -257,8 +256,8 @@ constexpr int GR_LCAP = 512;     // (leaf, mask) entries per warp
 struct GrShared {
   int code[GR_LCAP];       // leaf: pstart*8 + count-1
   unsigned mask[GR_LCAP];  // lanes whose walk opened the leaf
-  float4 fa[32];           // popped cells: hA32
-  float fh[32];            // hrm32
+  float4 fa[32];           // popped cells: centre, rmax
+  float fh[32];            // hrangemax
   unsigned fm[32];         // lanes whose walk reaches the cell
   int fc[32];
   int fu[32];              // popped cells the group test leaves undecided
@@ -326,7 +325,7 @@ __device__ __forceinline__ int gr_decide(const GrGroup& g, const float4& c, floa
 }
 
 // Walk for the lanes in `lanes`, appending the opened leaves to R.code/R.mask
-// from nent on.  gtest(hA32, hrm32) is the group test of a popped cell (1: it
+// from nent on.  gtest(centre and rmax, hrangemax) is the group test of a popped cell (1: it
 // passes for every lane, 2: for none, 0: undecided); test(e) is this lane's
 // test of undecided popped cell e (R.fa[e], R.fh[e], R.fc[e]).  Returns the
 // new entry count, or -1 when the list or the stack would overflow (nothing
@@ -729,7 +728,7 @@ __device__ __forceinline__ void gh_uv(int k, double& U, double& V) {
 // eight lanes read for one particle, and the sums they return.
 struct GpWarp {
   double x[32], y[32], z[32];
-  double hs[32], ih[32];           // (2h)^2 and 1/h of the pass in progress
+  double hs[32], ih[32];           // (2h)^2 (final pass) and 1/h of the pass in progress
   double part[32][4];
   int p[32], n[32], g[32];         // particle, candidates, gather neighbours
   int list[32];                    // the particles of the pass
@@ -806,7 +805,6 @@ __global__ void __launch_bounds__(GP_THREADS, 8) k_gradh_pass(
       const double ih = 1.0 / s.hp;                                    // :199-235
       const double hf = pow(ih, NDIMPR);
       W.ih[lane] = ih;
-      W.hs[lane] = (KERNRANGESQD * s.hp) * s.hp;
       if (active) W.list[__popc(A & lt)] = lane;
       const int na = __popc(A);
       __syncwarp();
@@ -2379,7 +2377,7 @@ inline int nb(long n, int t) { return (int)((n + t - 1) / t); }
 
 HydroTree hydro_tree(const Ctx& c) {
   const double delta = ldexp(1.0, -22) * (c.info.cellsize > 0.0 ? c.info.cellsize : 1.0);
-  return HydroTree{c.link, c.hA, c.hrm, c.hA32, c.hrm32, c.nkids, c.hN, c.info.ctot, c.info.root[0],
+  return HydroTree{c.link, c.hA, c.hrm, c.nkids, c.hN, c.info.ctot, c.info.root[0],
                    c.info.root[1], c.info.root[2], (float)delta, 0, c.info.rextent,
                    gh_unit(c.info.rextent), c.ncloud > 1 ? c.d_clouds : nullptr, c.ncloud};
 }
@@ -2625,13 +2623,11 @@ void launch_neib(Ctx& c, int nact, bool sorted) {
 //    to run: the gather part in the final pass's order, then the scatter part).
 // pptot ends as the full count in every row (the reference's pp_tot), and a
 // row of more than pp_limit neighbours keeps no list, as in the reference.
-// bitonic sort of N = 32 R values per warp, value r*32 + lane in e[r] (or,
-// with R = 1, of the first N <= 32 lanes' values, each block of N lanes on
-// its own, the first one ascending)
-template <int R, int N = 32 * R>
+// ascending bitonic sort of 32 R values per warp, value r*32 + lane in e[r]
+template <int R>
 __device__ __forceinline__ void warp_bitonic(int (&e)[R], int lane) {
 #pragma unroll
-  for (int size = 2; size <= N; size <<= 1) {
+  for (int size = 2; size <= 32 * R; size <<= 1) {
 #pragma unroll
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
       if (stride >= 32) {
@@ -2660,7 +2656,7 @@ __device__ __forceinline__ void warp_bitonic(int (&e)[R], int lane) {
   }
 }
 
-template <int R, int N = 32 * R>
+template <int R>
 __device__ __forceinline__ void sort_row(int* row, int m, int lane) {
   int e[R];
 #pragma unroll
@@ -2668,7 +2664,7 @@ __device__ __forceinline__ void sort_row(int* row, int m, int lane) {
     const int k = r * 32 + lane;
     e[r] = k < m ? row[k] : INT_MAX;
   }
-  warp_bitonic<R, N>(e, lane);
+  warp_bitonic(e, lane);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int k = r * 32 + lane;

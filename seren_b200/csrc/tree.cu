@@ -789,7 +789,7 @@ __device__ __forceinline__ void stock_cell(int c, const int4* __restrict__ link,
                               double4* __restrict__ bbmina, double4* __restrict__ bbmaxa,
                               double rootx, double rooty, double rootz, double delta,
                               const int* __restrict__ nkids, float4* __restrict__ wA,
-                              float4* __restrict__ hA32, float4* __restrict__ hN,
+                              float4* __restrict__ hN,
                               const double* __restrict__ hrm,
                               const CloudInfo* __restrict__ cl, int ncl) {
   const int4 lk = link[c];
@@ -905,7 +905,6 @@ __device__ __forceinline__ void stock_cell(int c, const int4* __restrict__ link,
   hA[c] = hn;
   const float4 h32 = make_float4((float)(hn.x - rootx), (float)(hn.y - rooty),
                                  (float)(hn.z - rootz), __double2float_ru(hn.w));
-  hA32[c] = h32;
   hN[2 * c] = h32;
   // (a restock leaves the cell's search range as it is, until the next hmax update)
   hN[2 * c + 1] = make_float4(__double2float_ru(hrm[c]), __int_as_float(lk.x > 0 ? lk.w : lk.z),
@@ -930,7 +929,6 @@ struct StockArgs {
   double rootx, rooty, rootz, delta;
   const int* nkids;
   float4* wA;
-  float4* hA32;
   float4* hN;
   const double* hrm;
   const CloudInfo* cl;
@@ -938,7 +936,7 @@ struct StockArgs {
 };
 __device__ __forceinline__ void stock_one(int c, const StockArgs& a) {
   stock_cell(c, a.link, a.pm, a.hz, a.thetamaxsqd, a.daux, a.gA, a.gB, a.gC, a.hA, a.hmaxa,
-             a.bbmina, a.bbmaxa, a.rootx, a.rooty, a.rootz, a.delta, a.nkids, a.wA, a.hA32, a.hN,
+             a.bbmina, a.bbmaxa, a.rootx, a.rooty, a.rootz, a.delta, a.nkids, a.wA, a.hN,
              a.hrm, a.cl, a.ncl);
 }
 __global__ void k_stock_level(int cfirst, int clast, StockArgs a) {
@@ -958,7 +956,7 @@ __global__ void __launch_bounds__(TOP_T) k_stock_top(int levels, LevelFirst F, S
 __device__ __forceinline__ void hmax_cell(int c, const int4* __restrict__ link,
                                           const int* __restrict__ nkids,
                                           const double2* __restrict__ hz, double* hrm,
-                                          float* __restrict__ hrm32, float4* __restrict__ hN) {
+                                          float4* __restrict__ hN) {
   const int4 lk = link[c];
   double hr = 0.0;
   if (lk.x > 0) {
@@ -968,24 +966,22 @@ __device__ __forceinline__ void hmax_cell(int c, const int4* __restrict__ link,
     for (int k = 0; k < nk; ++k) hr = fmax(hr, hrm[lk.z + k]);
   }
   hrm[c] = hr;
-  hrm32[c] = __double2float_ru(hr);
-  reinterpret_cast<float*>(hN)[8 * (size_t)c + 4] = hrm32[c];
+  reinterpret_cast<float*>(hN)[8 * (size_t)c + 4] = __double2float_ru(hr);
 }
 __global__ void k_hmax_level(int cfirst, int clast, const int4* __restrict__ link,
                              const int* __restrict__ nkids, const double2* __restrict__ hz,
-                             double* hrm, float* __restrict__ hrm32, float4* __restrict__ hN) {
+                             double* hrm, float4* __restrict__ hN) {
   const int c = cfirst + blockIdx.x * blockDim.x + threadIdx.x;
-  if (c <= clast) hmax_cell(c, link, nkids, hz, hrm, hrm32, hN);
+  if (c <= clast) hmax_cell(c, link, nkids, hz, hrm, hN);
 }
 __global__ void __launch_bounds__(TOP_T) k_hmax_top(int levels, LevelFirst F,
                                                     const int4* __restrict__ link,
                                                     const int* __restrict__ nkids,
                                                     const double2* __restrict__ hz, double* hrm,
-                                                    float* __restrict__ hrm32,
                                                     float4* __restrict__ hN) {
   for (int l = levels - 1; l >= 0; --l) {
     for (int c = F.first[l] + threadIdx.x; c < F.first[l + 1]; c += TOP_T)
-      hmax_cell(c, link, nkids, hz, hrm, hrm32, hN);
+      hmax_cell(c, link, nkids, hz, hrm, hN);
     __syncthreads();
   }
 }
@@ -1362,7 +1358,7 @@ void launch_stock(Ctx& c) {
   const double delta = ldexp(1.0, -22) * (c.info.cellsize > 0.0 ? c.info.cellsize : 1.0);
   const StockArgs a{c.link, c.pm, c.hz, c.prm.thetamaxsqd, daux, c.gA, c.gB, c.gC, c.hA, c.hmax,
                     c.bbmin, c.bbmax, c.info.root[0], c.info.root[1], c.info.root[2], delta,
-                    c.nkids, c.wA, c.hA32, c.hN, c.hrm, c.ncloud > 1 ? c.d_clouds : nullptr,
+                    c.nkids, c.wA, c.hN, c.hrm, c.ncloud > 1 ? c.d_clouds : nullptr,
                     c.ncloud};
   const int top = top_levels(c);
   for (int l = c.info.ltot; l >= top; --l) {
@@ -1378,11 +1374,11 @@ void launch_update_hmax(Ctx& c) {
   for (int l = c.info.ltot; l >= top; --l) {
     const int f = c.info.first_cell[l], la = c.info.last_cell[l];
     k_hmax_level<<<nb(la - f + 1, 128), 128, 0, c.st>>>(f, la, c.link, c.nkids, c.hz, c.hrm,
-                                                        c.hrm32, c.hN); ++c.nlaunch;
+                                                        c.hN); ++c.nlaunch;
   }
   if (top == 0) return;
   k_hmax_top<<<1, TOP_T, 0, c.st>>>(top, level_first(c, top), c.link, c.nkids, c.hz, c.hrm,
-                                    c.hrm32, c.hN); ++c.nlaunch;
+                                    c.hN); ++c.nlaunch;
 }
 
 void launch_hguess(Ctx& c) {
