@@ -6,11 +6,11 @@
 // Cells use the reference's breadth-first numbering (BHgrav_build.F90:149-157).
 //
 // This translation unit family is compiled with -fmad=false: every FP64
-// expression that mirrors a Fortran statement is evaluated with the same
-// association and no contraction, so integer decisions taken from floats
-// (octants, MAC tests, kernel bins, neighbour tests) agree with the FP64
-// reference arithmetic.  Kernels that want FMA (the mixed-precision pair
-// arithmetic) call fmaf()/fma() explicitly.
+// expression that an integer decision is taken from (octants, MAC tests, kernel
+// bins, neighbour tests), and the stock, is evaluated with the Fortran's
+// association and no contraction, so those decisions agree with the FP64
+// reference arithmetic.  Kernels that want FMA (the gravity terms, the sums of the
+// grad-h passes, the mixed-precision pair arithmetic) call fmaf()/fma() explicitly.
 #pragma once
 
 #include <cstdint>

@@ -53,7 +53,7 @@ __device__ __forceinline__ void cell_term64(double d0, double d1, double d2, dou
 
 // gravity/gravity_gradh.F90:11-95, d = r_q - r_p, zz = zeta/h^2 of each side, mh
 // = m_q/2.  r = sqrt(r^2) + SMALL_NUMBER and 1/r come from one rsqrt: the root
-// corrected by its residual, the SMALL_NUMBER to first order (below 1e-12,
+// corrected by its residual (one Newton step), the SMALL_NUMBER to first order (below 1e-12,
 // where that would not do, from the reference's own expressions).
 __device__ __forceinline__ void pair_term64(double d0, double d1, double d2, double ihp,
                                             double zzp, double mh, double hq, double ihq,
@@ -1114,8 +1114,11 @@ int grav_walk_slots(const Ctx& c) {
 // group gives each particle more lanes and a shorter list.  Measured with
 // groups of 32 / 16 / 8 / 4 (us): 777 particles FP64 229 / 135 / 90 / 63, 32768 FP64
 // 639 / 496 / 430 / 461, 50000 mixed 559 / 344 / 385 / 485, 200003 mixed 1325 / 1327 /
-// 1633 / 2273.  It depends on the cloud's size alone, so a cloud has the same
-// groups, and so the same sums bit for bit, alone and in a forest.
+// 1633 / 2273.  The width follows the number of particles walked (the active ones
+// of a list), in a forest the size of the cloud, not of the forest, and not the
+// precision: so a cloud has the same groups, and the same sums bit for bit, alone
+// and in a forest.  A forest of many small clouds pays for that (64 clouds of 4096,
+// mixed, ms: 0.77 / 0.87 / 1.13 / 1.63).
 int grav_lpw(int n) { return n <= 4096 ? 2 : n <= 16384 ? 3 : n <= 65536 ? 4 : 5; }
 
 int grav_walk_stack_cap(const Ctx& c) { return std::min(GW_STACK, c.cmax + 1); }

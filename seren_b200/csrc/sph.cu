@@ -2,13 +2,15 @@
 // hydro forces with MON97 viscosity, and the isothermal equation of state.
 //
 // grad-h and the neighbour lists run on group walks: a warp walks the tree
-// for 32 neighbouring particles at once with each lane's own test, so every
+// for up to 32 neighbouring particles at once with each lane's own test, so every
 // lane opens exactly the leaves of its own reference walk (BHhydrowalk_hgather,
-// BHhydro_walk); the lanes then run their reference routines over the shared
-// list of opened leaves.  Neighbour lists come out in the reference's order
-// (depth-first leaf order, particles in leaf order); density sums only differ
-// from the reference's in the order of their terms.  The hydro force kernel
-// gives one thread to one particle and follows hydro_gradh step by step.
+// BHhydro_walk).  grad-h records each particle's candidates from those leaves and
+// iterates over them; neighbour lists follow from the gather sets of its final
+// passes, or from a walk of their own, and come out in the reference's order
+// (depth-first leaf order, particles in leaf order) when the caller reads them.
+// Density sums differ from the reference's in the order of their terms and by
+// fused multiply-adds.  The hydro force kernel gives a few threads to a particle,
+// which share out its list.
 #include <algorithm>
 #include <climits>
 #include <mutex>
@@ -698,8 +700,11 @@ __device__ __forceinline__ int gp_flatten(const int* __restrict__ row, int n, in
 }
 
 // The kernel bin int(5000 r/h) of a pair, y = (r/h)^2, from an FP32 root; sure =
-// false when that lies too close to a bin's edge to tell (its error is below
-// 2e-3 bins; y not a normal FP32 number included) and gh_bin_exact must decide.
+// false when that lies too close to a bin's edge to tell (y not a normal FP32 number
+// included) and gh_bin_exact must decide.  Its relative error is at most 2^-24 for
+// the roundings of y and t2 together under the root, 2^-22.9 for rsqrt.approx and
+// 2^-24 for the last product, 2.5e-7 in all: 2.5e-3 bins at 2h (bin 10^4), and within
+// the 4e-3 kept free at a bin's edges up to 1.6e4 bins.
 __device__ __forceinline__ int gh_bin(double y, bool& sure) {
   const float t2 = (float)y * 2.5e7f;
   const float t = t2 * rsqrt_n(t2);
@@ -740,7 +745,9 @@ struct GpWarp {
 // time.  A warp takes 2^lpw particles: fewer when there are too few for every
 // resident warp to get 32 (a particle's sums do not depend on it).
 //
-// Bound by the latency of its gathers and FP64 chains.  On a 1M-particle core: 1.45
+// Bound by the latency of its gathers and FP64 chains, part of it perhaps that of
+// its own spills (228 bytes stored, 336 loaded at 64 registers; a form for 6 blocks
+// per SM took 1.8 ms).  On a 1M-particle core: 1.45
 // ms (3.13 ms when a warp took one particle at a time, tested every particle of
 // its opened leaves and packed those in range before evaluating them); with
 // k_gradh_walk, which now does the testing (0.92 ms before), 3.0 ms against 4.05.
@@ -2090,9 +2097,6 @@ __device__ __forceinline__ float m4_w1_bin(float x, bool tc) {
 constexpr int HY_SUB = 4;        // threads per particle in the mixed hydro kernel
 constexpr int HY_SUB64 = 8;      // and in the FP64 one (1M core: 1.82 ms with 1, 1.45 with 4 or 8; 777: 132, 52, 39 us)
 
-// SUB consecutive threads share one particle, each taking every SUB-th entry
-// of its neighbour list, and their sums are added at the end (SUB = 1 keeps the
-// reference's order of terms).
 // k_hydro_prep for the mixed kernel, which also writes the neighbours' values
 // as one 96-byte record per particle (three 32-byte sectors: x, y, z, m |
 // vx, vy, vz, h | pf, hf4, c_s, rho), so that a pair gathers two or three
@@ -2310,8 +2314,11 @@ struct HydroSum {
   }
 };
 
-// A particle whose neighbours outnumber its list (pptot > pp_limit) goes to over /
-// nover, for k_hydro_over; without them (the form without a context) there is none.
+// SUB consecutive threads share one particle, each taking every SUB-th entry
+// of its neighbour list, and their sums are added at the end.  A particle whose
+// neighbours outnumber its list (pptot > pp_limit) goes to over / nover, for
+// k_hydro_over; without them (the form without a context) there is none.  (At 64
+// registers the FP64 form spills 64 bytes.)
 template <bool MIXED, int SUB, bool PACKED = false>
 __global__ void __launch_bounds__(128, 8) k_hydro(int nact, const int* __restrict__ act,
                                                HydroArrays A, const int* __restrict__ pptot,
@@ -2476,7 +2483,9 @@ void launch_gradh(Ctx& c, int nact) {
       c.prm.pp_gather, c.info.rextent, c.leaves, c.nleaf, c.npot, c.redo, c.work + 1,
       c.pplist, c.prm.pp_limit, c.d_err, counts, c.work, t.cl, t.ncl, rec ? 1 : 0, c.pptot);
   // three walk buffers of wstack_cap entries per redo warp (a walk-stack slot holds
-  // two), for as many warps as fit or as there are buffers for
+  // two), for as many warps as fit or as there are buffers for: half the length and
+  // twice the warps of one slot per buffer (first call of a 200k core 6.2 ms of
+  // grad-h, 8.0 before); walks of more entries go on in the whole-GPU rounds
   static int rocc[16] = {};
   int& ro = rocc[c.dev >= 0 && c.dev < 16 ? c.dev : 0];
   if (ro == 0) {
@@ -2780,7 +2789,9 @@ __device__ __forceinline__ void neib_visit(int p, int q, const float4& F, const 
 // put in increasing order.  Neither reads what the other writes: a walked row
 // takes no scatter entries.  (As kernels of their own, the few walks were 50 us of
 // latency each.)  Bound by the latency of the record gathers, so 8 blocks per SM: 4M
-// core 1.67 ms, 2.02 at 6, 1.97 with FP64 records of 32 bytes.
+// core 1.67 ms, 2.02 at 6, 1.97 with FP64 records of 32 bytes.  That leaves 32
+// registers, and the walk spills (256 bytes stored, 284 loaded): where every
+// particle is listed, 16 us per 1000 of them against 12 in a kernel of its own.
 constexpr int NT_THREADS = 256;
 constexpr int NT_WARPS = NT_THREADS / 32;
 constexpr int NT_SEG = 8;        // (little shared memory: the gathers live on L1)

@@ -1125,8 +1125,7 @@ size_t radix_hist_ints(size_t pmax) {
 }
 
 // stable sort of (keys, idx) on the key bits [lo, bits), 8 at a time; an even
-// number of passes leaves the sorted data in keys/idx.  Few items: one block
-// sorts on all bits (idx holds the input order of equal keys in increasing order).
+// number of passes leaves the sorted data in keys/idx
 static void radix_sort(Ctx& c, int n, int lo, int bits) {
   if (n < RS_SMALL) radix_passes<4>(c, n, lo, bits);
   else radix_passes<16>(c, n, lo, bits);
