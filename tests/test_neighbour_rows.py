@@ -12,25 +12,57 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("kind,n", [("plummer", 20001), ("disc", 5003)])
-def test_force_step_repeats_bit_for_bit(kind, n, precision):
-    """Scatter parts of more and fewer than 16 entries, overflowed rows, redone
-    particles: the same input gives the same bits."""
+@pytest.mark.parametrize("kind,n,pp_limit", [
+    ("plummer", 20001, None), ("disc", 5003, None), ("plummer", 20001, 60), ("disc", 5003, 60)])
+def test_force_step_repeats_bit_for_bit(kind, n, pp_limit, precision):
+    """The same input gives the same bits, and in FP64 the oracle's numbers; with
+    scatter parts of more and fewer than 16 entries, redone particles, and rows
+    that overflow pp_limit."""
     from seren_b200.gpu import GpuHotPath
     ic = (ics.plummer if kind == "plummer" else ics.protostellar_disc)(n=n, seed=61)
+    ic["sound"] = np.full(n, 0.1)
+    prm = params(ic, precision=precision)
+    if pp_limit:
+        prm.pp_limit = pp_limit
     first = None
     for _ in range(3):
-        g = GpuHotPath(n, params(ic, precision=precision))
+        g = GpuHotPath(n, prm)
         out = g.force_step_io(ic["parray"], ic["v"], ic["sound"] ** 2, first_call=True)
+        assert g.last_step_stats()[2][15] > 0               # particles redone
         out = g.force_step_io(out["parray"], out["v"], out["csq"])
         g.close()
         if first is None:
             first = out
         for k in first:
             assert np.array_equal(first[k], out[k]), k
+    # the oracle's second evaluation, and what its lists hold
+    o = Oracle(n, params(ic))
+    p, perm = o.tree_update(ic["parray"])
+    s = o.sph_update(p, ic["v"][perm], first_call=True)
+    v = ic["v"][perm]
+    p, perm = o.tree_update(s["parray"])
+    v = v[perm]
+    s = o.sph_update(p, v)
+    sound = np.full(n, 0.1)
+    a, _ = o.grav_forces(o.hydro_forces(sound * sound * s["rho"], sound))
+    o.close()
+    p, tot = s["parray"], s["pptot"]
+    if kind == "plummer" or pp_limit:
+        assert (tot > prm.pp_limit).any()                   # rows without a list
+    short = np.flatnonzero(tot <= prm.pp_limit)
+    scatter = np.zeros(n, int)                              # neighbours beyond a row's own 2h
+    for i in short:
+        d = p[s["pplist"][i, :tot[i]], 0:3] - p[i, 0:3]
+        scatter[i] = np.count_nonzero((d * d).sum(axis=1) > 4.0 * p[i, 4] ** 2)
+    assert (scatter > 16).any() and ((scatter > 0) & (scatter <= 16)).any()
+    if precision == 0:
+        # FP64 sums of some hundred terms in another order
+        assert rel_rows(first["rho"], s["rho"]).max() < 1e-11
+        assert rel_rows(first["a"], a).max() < 1e-9
 
 
-@pytest.mark.parametrize("n,nsink", [(37, 1), (5000, 3), (5000, 200)])
+# (100003 particles: the walks' scratch takes the 1000 sinks in two rounds)
+@pytest.mark.parametrize("n,nsink", [(37, 1), (5000, 3), (5000, 200), (100003, 1000)])
 def test_sink_forces_of_many_sinks(n, nsink):
     from seren_b200.gpu import GpuHotPath
     ic = ics.plummer(n=n, seed=62)
