@@ -745,9 +745,9 @@ struct GpWarp {
 // time.  A warp takes 2^lpw particles: fewer when there are too few for every
 // resident warp to get 32 (a particle's sums do not depend on it).
 //
-// Bound by the latency of its gathers and FP64 chains, part of it perhaps that of
-// its own spills (228 bytes stored, 336 loaded at 64 registers; a form for 6 blocks
-// per SM took 1.8 ms).  On a 1M-particle core: 1.45
+// Bound by the latency of its gathers and FP64 chains (at 64 registers it spills 228
+// bytes, 1.4 % of its instructions; a form for 6 blocks per SM took 1.8 ms).  On a
+// 1M-particle core: 1.45
 // ms (3.13 ms when a warp took one particle at a time, tested every particle of
 // its opened leaves and packed those in range before evaluating them); with
 // k_gradh_walk, which now does the testing (0.92 ms before), 3.0 ms against 4.05.
@@ -980,6 +980,9 @@ __global__ void __launch_bounds__(GP_THREADS, 8) k_gradh_pass(
 // warp in the walk stacks, idle while this kernel runs), and the passes flatten
 // the leaves GP_SEG at a time and share the candidates out over the lanes.  The
 // final pass records the gather neighbours (rec) as k_gradh_pass does.
+// A particle whose walk outgrows the buffers is listed with its state in its row, for
+// the whole-GPU rounds; or, when they are many, for a second round here (resume)
+// with buffers twice as long, which starts from the walk they stopped at.
 constexpr int RD_THREADS = 128;
 constexpr int RD_WARPS = RD_THREADS / 32;
 
@@ -1108,7 +1111,7 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
     HydroTree t, const double4* __restrict__ tabA, double h_fac, int pp_gather, double rextent0,
     int* __restrict__ scratch, int cap, int* __restrict__ wide, int* __restrict__ nwide,
     int* __restrict__ leaves, const int* __restrict__ nrow, int* __restrict__ npot,
-    int* __restrict__ gset, int L, int rec, int* __restrict__ pptot, DevError* err,
+    int* __restrict__ gset, int L, int rec, int* __restrict__ pptot, int resume, DevError* err,
     unsigned long long* counts) {
   __shared__ int cand_all[RD_WARPS][GP_SEG * LEAFMAX];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1142,7 +1145,11 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
     };
     int nl = 0;
     const int* lf = lv;
-    if (const int row = nrow[p]; row < -1) {           // walked at h*HMULT (:154-170)
+    bool pending = false;                              // the walk at h_high still to be made
+    if (resume) {
+      s = *reinterpret_cast<const GhState*>(leaves + (size_t)p * GH_LEAVES);
+      pending = true;
+    } else if (const int row = nrow[p]; row < -1) {    // walked at h*HMULT (:154-170)
       lf = leaves + (size_t)p * GH_LEAVES;
       nl = -1 - row;
       s.h_high = s.hp * HMULT;
@@ -1151,8 +1158,9 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
     bool over = false, bad = false;
     while (true) {
       while (true) {                                                   // :154-191
-        if (s.hp > s.h_high) {
-          s.h_high = s.hp * HMULT;
+        if (pending || s.hp > s.h_high) {
+          if (!pending) s.h_high = s.hp * HMULT;
+          pending = false;
           Rw = KERNRANGE * s.h_high;
           R32 = (float)Rw;
           int cnt = 0;
@@ -1195,7 +1203,7 @@ __global__ void __launch_bounds__(RD_THREADS) k_gradh_redo(
       continue;
     }
     if (over) {                                        // more than cap leaves or cells a level
-      // the whole-GPU path takes the particle from here: its state goes to
+      // the next round takes the particle from here: its state goes to
       // its row (no longer read once the particle has walked again), and its
       // next step is the counting walk at s.h_high that outgrew the scratch
       if (lane == 0) {
@@ -2482,27 +2490,46 @@ void launch_gradh(Ctx& c, int nact) {
       ngrp, gl, lpw, c.pm, c.hz, c.vel, c.rho, c.omega, c.div_v, c.drhodt, c.tabA, c.prm.h_fac,
       c.prm.pp_gather, c.info.rextent, c.leaves, c.nleaf, c.npot, c.redo, c.work + 1,
       c.pplist, c.prm.pp_limit, c.d_err, counts, c.work, t.cl, t.ncl, rec ? 1 : 0, c.pptot);
-  // three walk buffers of wstack_cap entries per redo warp (a walk-stack slot holds
-  // two), for as many warps as fit or as there are buffers for: half the length and
-  // twice the warps of one slot per buffer (first call of a 200k core 6.2 ms of
-  // grad-h, 8.0 before); walks of more entries go on in the whole-GPU rounds
+  // three walk buffers per redo warp: of wstack_cap entries (half a walk-stack slot)
+  // each, for as many warps as fit or as there are buffers for (first call of a 200k
+  // core 6.2 ms of grad-h, 8.0 with buffers of a slot).  When more particles outgrow
+  // them than a batch of whole-GPU rounds takes, a second round with buffers of a slot
+  // and half the warps takes what it can: it costs the latency of one warp's longest
+  // walk, and each batch it saves tens of ms.  First calls, grad-h in ms, without and
+  // with it: 300k disc (49 such particles) 10.2 / 12.9, 200k core at h_fac 2.5 (733)
+  // 26.3 / 27.0; 1M core at 1.7 (1531) 84.7 / 71.6, 2M disc (1792) 117 / 86, 4M disc
+  // (4355) 347 / 243.
   static int rocc[16] = {};
   int& ro = rocc[c.dev >= 0 && c.dev < 16 ? c.dev : 0];
   if (ro == 0) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ro, k_gradh_redo, RD_THREADS, 0);
     if (ro < 1) ro = 1;
   }
-  const int rblocks = std::min(sm_count(c) * ro, (2 * c.wstack_slots / 3) / RD_WARPS);
-  k_gradh_redo<<<std::max(1, rblocks), RD_THREADS, 0, c.st>>>(
-      c.redo, c.work + 1, c.pm, c.hz, c.vel, c.rho, c.omega, c.div_v, c.drhodt, t, c.tabA,
-      c.prm.h_fac, c.prm.pp_gather, c.info.rextent, reinterpret_cast<int*>(c.wstack),
-      c.prm.redo_cap > 0 ? std::min(c.prm.redo_cap, c.wstack_cap) : c.wstack_cap,
-      c.wide, c.work + 2, c.leaves, c.nleaf, c.npot, c.pplist, c.prm.pp_limit, rec ? 1 : 0,
-      c.pptot, c.d_err, counts);
-  // the particles whose walks outgrew the redo kernel's scratch: rounds of
-  // whole-GPU walks until each has taken its last step
+  const int cap2 = c.prm.redo_cap > 0 ? std::min(c.prm.redo_cap, 2 * c.wstack_cap) : 2 * c.wstack_cap;
+  const int cap1 = (cap2 + 1) / 2;
+  auto redo = [&](int blocks, int cap, int resume, const int* list, const int* nlist, int* out,
+                  int* nout) {
+    k_gradh_redo<<<std::max(1, blocks), RD_THREADS, 0, c.st>>>(
+        list, nlist, c.pm, c.hz, c.vel, c.rho, c.omega, c.div_v, c.drhodt, t, c.tabA,
+        c.prm.h_fac, c.prm.pp_gather, c.info.rextent, reinterpret_cast<int*>(c.wstack), cap, out,
+        nout, c.leaves, c.nleaf, c.npot, c.pplist, c.prm.pp_limit, rec ? 1 : 0, c.pptot, resume,
+        c.d_err, counts);
+    ++c.nlaunch;
+  };
+  redo(std::min(sm_count(c) * ro, (2 * c.wstack_slots / 3) / RD_WARPS), cap1, 0, c.redo, c.work + 1,
+       c.wide, c.work + 2);
   int nwide = 0;
+  const int* wide = c.wide;
   read_dev(c, c.work + 2, &nwide, sizeof(int));
+  if (nwide > WD_BATCH) {
+    cudaMemsetAsync(c.work + 1, 0, sizeof(int), c.st);
+    redo(std::min(sm_count(c) * ro, (c.wstack_slots / 3) / RD_WARPS), cap2, 1, c.wide, c.work + 2,
+         c.redo, c.work + 1);
+    read_dev(c, c.work + 1, &nwide, sizeof(int));
+    wide = c.redo;
+  }
+  // the particles whose walks outgrew that scratch: rounds of whole-GPU walks until
+  // each has taken its last step
   if (nwide > 0) {
     const int round_cap = 4 * GRADH_ITERATION_MAX + 2 * HGROW_CAP + 16;
     const int nbrute = nb(c.ptot, WD_THREADS * BR_Q);
@@ -2544,7 +2571,7 @@ void launch_gradh(Ctx& c, int nact) {
     read_dev(c, c.scan.total, &ncover, sizeof(int));
     for (int b0 = 0; b0 < nwide; b0 += WD_BATCH) {
       const int n = std::min(WD_BATCH, nwide - b0);
-      k_wide_init<<<nb(n, 128), 128, 0, c.st>>>(n, c.wide + b0, c.pm, c.leaves, c.vel,
+      k_wide_init<<<nb(n, 128), 128, 0, c.st>>>(n, wide + b0, c.pm, c.leaves, c.vel,
                                                   c.info.rextent, c.ptot, t.cl, t.ncl,
                                                   static_cast<WideState*>(c.wst), c.wacc, counts);
       ++c.nlaunch;
@@ -2576,7 +2603,7 @@ void launch_gradh(Ctx& c, int nact) {
       }
     }
   }
-  c.nlaunch += 3;
+  c.nlaunch += 2;
   c.gsets = rec;
 }
 

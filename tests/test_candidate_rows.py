@@ -4,17 +4,17 @@ against the oracle."""
 import numpy as np
 import pytest
 
-from helpers import lists_equal, params, rel_rows, run_pipeline
+from helpers import case, lists_equal, params, rel_rows, run_pipeline
 from oracle.oracle import Oracle
 from seren_b200 import ics
 
 pytestmark = pytest.mark.gpu
 
 
-def _compare(ic, first_call):
+def _compare(ic, first_call, redo_cap=0):
     from seren_b200.gpu import GpuHotPath
     n = ic["parray"].shape[0]
-    g, o = GpuHotPath(n, params(ic)), Oracle(n, params(ic))
+    g, o = GpuHotPath(n, params(ic, redo_cap=redo_cap)), Oracle(n, params(ic))
     rg, ro = run_pipeline(g, ic, first_call), run_pipeline(o, ic, first_call)
     limit = g.params.pp_limit
     g.close()
@@ -87,3 +87,23 @@ def test_rows_that_overflow_are_not_walked_again(precision):
         s2 = o.sph_update(p2, ic["v"][perm][perm2])
         o.close()
         assert rel_rows(out[0]["rho"], s2["rho"]).max() < 1e-10
+
+
+@pytest.mark.parametrize("redo_cap", [60, 300])
+def test_redo_rounds(redo_cap):
+    """Walks that outgrow the redo kernel's first buffers (half of redo_cap) go on in
+    its second round when they are more than 1024, and those that outgrow these in
+    the whole-GPU rounds."""
+    from seren_b200.gpu import GpuHotPath
+    ic = case("clumps12k")
+    _compare(ic, True, redo_cap)
+    n = ic["parray"].shape[0]
+    wide = []
+    for cap in (redo_cap // 2, redo_cap):
+        g = GpuHotPath(n, params(ic, redo_cap=cap))
+        g.upload(ic["parray"], ic["v"], ic["sound"] ** 2)
+        g.force_step(first_call=True)
+        wide.append(g.last_step_stats()[2][8])
+        g.close()
+    assert wide[0] > 1024                                # outgrow the first buffers
+    assert 0 < wide[1] < wide[0]
