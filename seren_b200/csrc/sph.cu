@@ -626,17 +626,20 @@ __global__ void __launch_bounds__(GR_THREADS) k_gradh_walk(
         }
         nb = 0;
       }
-      // a row that overflows: the lane's opened leaves
-      const bool big = live && lane < PW && n > GH_LEAVES;
-      if (__any_sync(FULL, big)) {
+      // a row that overflows: its lane's opened leaves, one such row at a time
+      const unsigned big = __ballot_sync(FULL, live && lane < PW && n > GH_LEAVES);
+      for (unsigned todo = big; todo != 0u; todo &= todo - 1u) {
+        const int j = __ffs(todo) - 1;
+        int* const row = rows + (size_t)__shfl_sync(FULL, p, j) * GH_LEAVES;
         int k = 0;
-        for (int e = 0; e < nent; ++e) {
-          if (big && ((R.mask[e] >> lane) & 1u)) {
-            if (k < GH_LEAVES) out[k] = R.code[e];
-            ++k;
-          }
+        for (int e = lane; e - lane < nent; e += 32) {
+          const bool mine = e < nent && ((R.mask[e] >> j) & 1u);
+          const unsigned m = __ballot_sync(FULL, mine);
+          const int o = k + __popc(m & ((1u << lane) - 1u));
+          if (mine && o < GH_LEAVES) row[o] = R.code[e];
+          k += __popc(m);
         }
-        if (big) n = k <= GH_LEAVES ? -1 - k : -1;
+        if (lane == j) n = k <= GH_LEAVES ? -1 - k : -1;
       }
     }
     if (live && lane < PW) {
