@@ -324,6 +324,7 @@ int alloc_all(Ctx& c) {
   cudaMemset(c.d_err, 0, sizeof(DevError));
   cudaMemset(c.d_counts, 0, sizeof(int) * 32);
   cudaMemset(c.hrm, 0, sizeof(double) * C);
+  cudaMemset(c.hN, 0, sizeof(float4) * 2 * C);
   for (auto& e : c.ev)
     if (cudaEventCreate(&e) != cudaSuccess) return -1;
   // kernel tables

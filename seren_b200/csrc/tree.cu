@@ -790,7 +790,6 @@ __device__ __forceinline__ void stock_cell(int c, const int4* __restrict__ link,
                               double rootx, double rooty, double rootz, double delta,
                               const int* __restrict__ nkids, float4* __restrict__ wA,
                               float4* __restrict__ hN,
-                              const double* __restrict__ hrm,
                               const CloudInfo* __restrict__ cl, int ncl) {
   const int4 lk = link[c];
   if (cl) {                                  // a forest: the cell's own cloud's root box
@@ -906,9 +905,11 @@ __device__ __forceinline__ void stock_cell(int c, const int4* __restrict__ link,
   const float4 h32 = make_float4((float)(hn.x - rootx), (float)(hn.y - rooty),
                                  (float)(hn.z - rootz), __double2float_ru(hn.w));
   hN[2 * c] = h32;
-  // (a restock leaves the cell's search range as it is, until the next hmax update)
-  hN[2 * c + 1] = make_float4(__double2float_ru(hrm[c]), __int_as_float(lk.x > 0 ? lk.w : lk.z),
-                              __int_as_float(lk.x > 0 ? lk.x : -nkids[c]), 0.0f);
+  // the second half but its first word, the cell's search range: that stays as it is
+  // until the next hmax update
+  int* const node = reinterpret_cast<int*>(hN + 2 * (size_t)c + 1);
+  node[1] = lk.x > 0 ? lk.w : lk.z;
+  node[2] = lk.x > 0 ? lk.x : -nkids[c];
 }
 
 // The cells [cfirst, clast] of one level; or (levels > 1) the levels
@@ -930,14 +931,13 @@ struct StockArgs {
   const int* nkids;
   float4* wA;
   float4* hN;
-  const double* hrm;
   const CloudInfo* cl;
   int ncl;
 };
 __device__ __forceinline__ void stock_one(int c, const StockArgs& a) {
   stock_cell(c, a.link, a.pm, a.hz, a.thetamaxsqd, a.daux, a.gA, a.gB, a.gC, a.hA, a.hmaxa,
              a.bbmina, a.bbmaxa, a.rootx, a.rooty, a.rootz, a.delta, a.nkids, a.wA, a.hN,
-             a.hrm, a.cl, a.ncl);
+             a.cl, a.ncl);
 }
 __global__ void k_stock_level(int cfirst, int clast, StockArgs a) {
   const int c = cfirst + blockIdx.x * blockDim.x + threadIdx.x;
@@ -1357,7 +1357,7 @@ void launch_stock(Ctx& c) {
   const double delta = ldexp(1.0, -22) * (c.info.cellsize > 0.0 ? c.info.cellsize : 1.0);
   const StockArgs a{c.link, c.pm, c.hz, c.prm.thetamaxsqd, daux, c.gA, c.gB, c.gC, c.hA, c.hmax,
                     c.bbmin, c.bbmax, c.info.root[0], c.info.root[1], c.info.root[2], delta,
-                    c.nkids, c.wA, c.hN, c.hrm, c.ncloud > 1 ? c.d_clouds : nullptr,
+                    c.nkids, c.wA, c.hN, c.ncloud > 1 ? c.d_clouds : nullptr,
                     c.ncloud};
   const int top = top_levels(c);
   for (int l = c.info.ltot; l >= top; --l) {
